@@ -9,78 +9,35 @@
 
 namespace rvf {
 
-// Separation of the centroid segment (a, b) and the triangle (p0, p1, p2)
-// along w, in FP32: true when the gap exceeds rm |w|.  Squares avoid the
-// square root (rm > 0).
-__device__ __forceinline__ bool axis_separates(const float* a, const float* b, const float4& p0, const float4& p1,
-                                               const float4& p2, float wx, float wy, float wz, float rm) {
-  const float sa = fmaf(a[0], wx, fmaf(a[1], wy, a[2] * wz)), sb = fmaf(b[0], wx, fmaf(b[1], wy, b[2] * wz));
-  const float q0 = fmaf(p0.x, wx, fmaf(p0.y, wy, p0.z * wz));
-  const float q1 = fmaf(p1.x, wx, fmaf(p1.y, wy, p1.z * wz));
-  const float q2 = fmaf(p2.x, wx, fmaf(p2.y, wy, p2.z * wz));
-  const float gap = fmaxf(fminf(q0, fminf(q1, q2)) - fmaxf(sa, sb), fminf(sa, sb) - fmaxf(q0, fmaxf(q1, q2)));
-  return gap > 0.0f && gap * gap > rm * rm * fmaf(wx, wx, fmaf(wy, wy, wz * wz));
-}
-
 // True when no ray of the pair (segments within R of the centroid segment
-// a -> b, direction d) can be a hit of the reference's test of the triangle
+// a -> a + d) can be a hit of the reference's test of the triangle
 // with corners p0, p1, p2 (FP32) and rounding margin p0.w.  em absorbs the
 // FP32 rounding of the corners and of this test (a few 2^-24 of the
 // coordinates' magnitude, against em = S 2^-16).
-__device__ __forceinline__ bool pair_misses_tri(const float* a, const float* b, const float* d, float R, float em,
-                                                const float4& p0, const float4& p1, const float4& p2) {
-  const float rm = R + p0.w + em;
-  const float f1[3] = {p1.x - p0.x, p1.y - p0.y, p1.z - p0.z};
-  const float f2[3] = {p2.x - p0.x, p2.y - p0.y, p2.z - p0.z};
-  const float f3[3] = {p2.x - p1.x, p2.y - p1.y, p2.z - p1.z};
-  // the segment direction crossed with each edge, then the triangle's normal
-  if (axis_separates(a, b, p0, p1, p2, d[1] * f1[2] - d[2] * f1[1], d[2] * f1[0] - d[0] * f1[2],
-                     d[0] * f1[1] - d[1] * f1[0], rm))
-    return true;
-  if (axis_separates(a, b, p0, p1, p2, d[1] * f2[2] - d[2] * f2[1], d[2] * f2[0] - d[0] * f2[2],
-                     d[0] * f2[1] - d[1] * f2[0], rm))
-    return true;
-  if (axis_separates(a, b, p0, p1, p2, d[1] * f3[2] - d[2] * f3[1], d[2] * f3[0] - d[0] * f3[2],
-                     d[0] * f3[1] - d[1] * f3[0], rm))
-    return true;
-  return axis_separates(a, b, p0, p1, p2, f1[1] * f2[2] - f1[2] * f2[1], f1[2] * f2[0] - f1[0] * f2[2],
-                        f1[0] * f2[1] - f1[1] * f2[0], rm);
-}
-
-// The same test over more separating axes: the coordinate axes first (the
-// cheapest and, for the long thin triangles the reference's transposed read
-// produces, often enough), then the segment direction crossed with each
-// edge, the normal, and each coordinate axis crossed with each edge.  Each
-// axis is a valid separation on its own (the capsule projects onto w as its
-// centroid segment widened by rm |w|), so more axes only drop more.
-__device__ __forceinline__ bool pair_misses_tri_full(const float* a, const float* b, const float* d, float R,
-                                                     float em, const float4& p0, const float4& p1,
-                                                     const float4& p2) {
-  const float rm = R + p0.w + em;
-  {
-    const float ax[3] = {a[0], a[1], a[2]}, bx[3] = {b[0], b[1], b[2]};
-    const float q0[3] = {p0.x, p0.y, p0.z}, q1[3] = {p1.x, p1.y, p1.z}, q2[3] = {p2.x, p2.y, p2.z};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float tlo = fminf(q0[k], fminf(q1[k], q2[k])), thi = fmaxf(q0[k], fmaxf(q1[k], q2[k]));
-      const float slo = fminf(ax[k], bx[k]), shi = fmaxf(ax[k], bx[k]);
-      if (tlo - shi > rm || slo - thi > rm) return true;
-    }
-  }
-  if (pair_misses_tri(a, b, d, R, em, p0, p1, p2)) return true;
-  const float f[3][3] = {{p1.x - p0.x, p1.y - p0.y, p1.z - p0.z},
-                         {p2.x - p0.x, p2.y - p0.y, p2.z - p0.z},
-                         {p2.x - p1.x, p2.y - p1.y, p2.z - p1.z}};
-#pragma unroll
-  for (int m = 0; m < 3; ++m)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      float w[3] = {0.f, 0.f, 0.f};  // e_k x f_m
-      w[(k + 1) % 3] = -f[m][(k + 2) % 3];
-      w[(k + 2) % 3] = f[m][(k + 1) % 3];
-      if (axis_separates(a, b, p0, p1, p2, w[0], w[1], w[2], rm)) return true;
-    }
-  return false;
+__device__ __forceinline__ bool pair_misses_tri(const float* a, const float* d, float R, float em, const float4& p0,
+                                                const float4& p1, const float4& p2) {
+  const float rm = R + p0.w + em, rm2 = rm * rm;
+  const float s0[3] = {p0.x - a[0], p0.y - a[1], p0.z - a[2]};
+  const float s1[3] = {p1.x - a[0], p1.y - a[1], p1.z - a[2]};
+  const float s2[3] = {p2.x - a[0], p2.y - a[1], p2.z - a[2]};
+  // w = d x (edge g - e): the whole segment projects onto 0 (from a), both ends
+  // of the edge onto g.w, the third corner onto h.w
+  auto edge = [&](const float4& e, const float4& g, const float* sg, const float* sh) {
+    const float fx = g.x - e.x, fy = g.y - e.y, fz = g.z - e.z;
+    const float wx = d[1] * fz - d[2] * fy, wy = d[2] * fx - d[0] * fz, wz = d[0] * fy - d[1] * fx;
+    const float u = fmaf(sg[0], wx, fmaf(sg[1], wy, sg[2] * wz)), v = fmaf(sh[0], wx, fmaf(sh[1], wy, sh[2] * wz));
+    const float gap = fmaxf(fminf(u, v), -fmaxf(u, v));
+    return gap > 0.0f && gap * gap > rm2 * fmaf(wx, wx, fmaf(wy, wy, wz * wz));
+  };
+  if (edge(p0, p1, s0, s2)) return true;
+  if (edge(p0, p2, s0, s1)) return true;
+  if (edge(p1, p2, s1, s0)) return true;
+  // the triangle's normal: its plane at s0.n, the segment from 0 to d.n
+  const float f1[3] = {p1.x - p0.x, p1.y - p0.y, p1.z - p0.z}, f2[3] = {p2.x - p0.x, p2.y - p0.y, p2.z - p0.z};
+  const float nx = f1[1] * f2[2] - f1[2] * f2[1], ny = f1[2] * f2[0] - f1[0] * f2[2], nz = f1[0] * f2[1] - f1[1] * f2[0];
+  const float u = fmaf(s0[0], nx, fmaf(s0[1], ny, s0[2] * nz)), e = fmaf(d[0], nx, fmaf(d[1], ny, d[2] * nz));
+  const float gap = fmaxf(u - fmaxf(e, 0.0f), fminf(e, 0.0f) - u);
+  return gap > 0.0f && gap * gap > rm2 * fmaf(nx, nx, fmaf(ny, ny, nz * nz));
 }
 
 // The pair's capsule for the list walk, in FP32: the centroid segment's

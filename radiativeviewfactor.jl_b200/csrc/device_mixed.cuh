@@ -61,68 +61,59 @@ __device__ __forceinline__ bool make_ray_f(const float* xo, float rx, float ry, 
 // intervals overlaps: the comparison te <= tx of the reference.  An interval
 // never needs a margin against itself -- in particular the two ends of a
 // slab of zero thickness (lo == hi, as for the leaves of a flat face) are the
-// same number in FP32 and in FP64 -- so when te and tx are within the error
-// band the six pairs are checked one by one with margins.
+// same number in FP32 and in FP64 -- so each interval's end is compared with
+// the largest start of the others, and the smallest such slack decides.
 __device__ __forceinline__ int slab_f(const NodeF& nd, const RayF& R) {
-  float t1x = (nd.lo[0] - R.o[0]) * R.inv[0], t2x = (nd.hi[0] - R.o[0]) * R.inv[0];
-  float t1y = (nd.lo[1] - R.o[1]) * R.inv[1], t2y = (nd.hi[1] - R.o[1]) * R.inv[1];
-  float t1z = (nd.lo[2] - R.o[2]) * R.inv[2], t2z = (nd.hi[2] - R.o[2]) * R.inv[2];
+  const float t1x = (nd.lo[0] - R.o[0]) * R.inv[0], t2x = (nd.hi[0] - R.o[0]) * R.inv[0];
+  const float t1y = (nd.lo[1] - R.o[1]) * R.inv[1], t2y = (nd.hi[1] - R.o[1]) * R.inv[1];
+  const float t1z = (nd.lo[2] - R.o[2]) * R.inv[2], t2z = (nd.hi[2] - R.o[2]) * R.inv[2];
   const float lx = fminf(t1x, t2x), hx = fmaxf(t1x, t2x);
   const float ly = fminf(t1y, t2y), hy = fmaxf(t1y, t2y);
   const float lz = fminf(t1z, t2z), hz = fmaxf(t1z, t2z);
-  float te = fmaxf(fmaxf(fmaxf(lx, ly), lz), 0.0f);
-  float tx = fminf(fminf(fminf(hx, hy), hz), R.tmax);
-  float m = R.k0 + 2.0f * kRho * (fabsf(te) + fabsf(tx) + R.tmax);
-  if (te + m < tx) return kHit;
-  if (te > tx + m) return kMiss;
-  // pairwise overlaps of different intervals
-  const float lo[4] = {lx, ly, lz, 0.0f}, hi[4] = {hx, hy, hz, R.tmax};
-  bool unsure = false;
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      if (u == v) continue;
-      if (lo[u] > hi[v] + m) return kMiss;
-      if (!(lo[u] + m < hi[v])) unsure = true;
-    }
-  return unsure ? kUnsure : kHit;
+  const float xy = fmaxf(lx, ly), zs = fmaxf(lz, 0.0f);
+  const float te = fmaxf(xy, zs);
+  const float tx = fminf(fminf(fminf(hx, hy), hz), R.tmax);
+  const float m = R.k0 + 2.0f * kRho * (fabsf(te) + fabsf(tx) + R.tmax);
+  const float slack = fminf(fminf(hx - fmaxf(ly, zs), hy - fmaxf(lx, zs)),
+                            fminf(hz - fmaxf(xy, 0.0f), R.tmax - fmaxf(xy, lz)));
+  return slack > m ? kHit : slack < -m ? kMiss : kUnsure;
 }
 
 // Moller-Trumbore with certified outcome; the triangle stores |e1|, |e2|
-// (rounded up) in n1, n2.
+// (rounded up) in n1, n2.  The reference's u, v, t are quotients U / a, V / a,
+// T / a; with |a| certainly above its cut, each comparison is taken between
+// the numerators and multiples of |a| (no division), the numerators within
+//   |dU| <= (kE0 ns + d2) n2,  |dV| <= (kE0 ns + 2 d2) n1,  |dT| <= (kE0 ns + 2 d2) n1 n2
+// and |da| <= kE0 n1 n2 of the reference's (ns bounds |o - v0|, d2 = 2 delta;
+// the relative terms also cover its own FP64 rounding).
 __device__ __forceinline__ int mt_f(const TriF& t, const RayF& R) {
   const float n1 = __int_as_float(t.pad0), n2 = __int_as_float(t.pad1);
-  float hx = fmaf(R.d[1], t.e2[2], -R.d[2] * t.e2[1]);
-  float hy = fmaf(R.d[2], t.e2[0], -R.d[0] * t.e2[2]);
-  float hz = fmaf(R.d[0], t.e2[1], -R.d[1] * t.e2[0]);
-  float a = fmaf(t.e1[0], hx, fmaf(t.e1[1], hy, t.e1[2] * hz));
-  const float na = n1 * n2;
-  const float Ea = kE0 * na;
-  const float aa = fabsf(a);
-  if (aa + Ea < 1e-10f) return kMiss;
-  if (aa - Ea < 1e-10f) return kUnsure;
-  const float f = rcp_approx(a);
-  const float ia = fabsf(f);
-  float sx = R.o[0] - t.v0[0], sy = R.o[1] - t.v0[1], sz = R.o[2] - t.v0[2];
-  const float ns = fabsf(sx) + fabsf(sy) + fabsf(sz) + 2.0f * R.delta;
+  const float hx = fmaf(R.d[1], t.e2[2], -R.d[2] * t.e2[1]);
+  const float hy = fmaf(R.d[2], t.e2[0], -R.d[0] * t.e2[2]);
+  const float hz = fmaf(R.d[0], t.e2[1], -R.d[1] * t.e2[0]);
+  const float a = fmaf(t.e1[0], hx, fmaf(t.e1[1], hy, t.e1[2] * hz));
+  const float na = n1 * n2, Ea = kE0 * na;
+  const float aa = fabsf(a), hi = aa + Ea, lo = aa - Ea;
+  if (hi < 1e-10f) return kMiss;
+  if (lo < 1e-10f) return kUnsure;
+  const float sx = R.o[0] - t.v0[0], sy = R.o[1] - t.v0[1], sz = R.o[2] - t.v0[2];
   const float d2 = 2.0f * R.delta;
-  float u = f * fmaf(sx, hx, fmaf(sy, hy, sz * hz));
-  float Eu = fmaf(fabsf(u), Ea, (kE0 * ns + d2) * n2) * ia + kE0 * fabsf(u);
-  if (u < -Eu || u > 1.0f + Eu) return kMiss;
-  float qx = fmaf(sy, t.e1[2], -sz * t.e1[1]);
-  float qy = fmaf(sz, t.e1[0], -sx * t.e1[2]);
-  float qz = fmaf(sx, t.e1[1], -sy * t.e1[0]);
-  float v = f * fmaf(R.d[0], qx, fmaf(R.d[1], qy, R.d[2] * qz));
-  float Ev = fmaf(fabsf(v), Ea, (kE0 * ns + 2.0f * d2) * n1) * ia + kE0 * fabsf(v);
-  if (v < -Ev || u + v > 1.0f + Eu + Ev + 1e-6f) return kMiss;
-  float tt = f * fmaf(t.e2[0], qx, fmaf(t.e2[1], qy, t.e2[2] * qz));
-  float Et = fmaf(fabsf(tt), Ea, (kE0 * ns + 2.0f * d2) * na) * ia + kE0 * fabsf(tt);
-  const float Etm = Et + 2.0f * kRho * R.tmax;
-  if (tt < (float)kTEps - Et || tt > R.tmax + Etm) return kMiss;
-  const bool inside = (u > Eu && u < 1.0f - Eu) && (v > Ev && u + v < 1.0f - Eu - Ev - 1e-6f);
-  if (inside && tt > (float)kTEps + Et && tt < R.tmax - Etm) return kHit;
-  return kUnsure;
+  const float e = fmaf(kE0, fabsf(sx) + fabsf(sy) + fabsf(sz) + d2, d2), e2 = e + d2;
+  const float u = copysignf(1.0f, a) * fmaf(sx, hx, fmaf(sy, hy, sz * hz));
+  const float cu = e * n2;
+  if (u < -cu || u > hi + cu) return kMiss;
+  const float qx = fmaf(sy, t.e1[2], -sz * t.e1[1]);
+  const float qy = fmaf(sz, t.e1[0], -sx * t.e1[2]);
+  const float qz = fmaf(sx, t.e1[1], -sy * t.e1[0]);
+  const float v = copysignf(1.0f, a) * fmaf(R.d[0], qx, fmaf(R.d[1], qy, R.d[2] * qz));
+  const float cv = e2 * n1, cuv = cu + cv + 1e-6f * aa;
+  if (v < -cv || u + v > hi + cuv) return kMiss;
+  const float w = copysignf(1.0f, a) * fmaf(t.e2[0], qx, fmaf(t.e2[1], qy, t.e2[2] * qz));
+  const float cw = e2 * na;
+  const float eps = (float)kTEps, tm = 2.0f * kRho * R.tmax;
+  if (w + cw < (1.0f - kE0) * eps * lo || w - cw > (R.tmax + tm) * hi) return kMiss;
+  const bool inside = u > cu && u < lo - cu && v > cv && u + v < lo - cuv;
+  return inside && w - cw > (1.0f + kE0) * eps * hi && w + cw < (R.tmax - tm) * lo ? kHit : kUnsure;
 }
 
 // Warp-coherent FP32 any-hit traversal (same walk as packet_any_hit) with

@@ -75,7 +75,7 @@ struct TileClassArgs {
   const float4* sat;
   float sat_em;
   uint8_t* cls;    // n_tiles
-  uint32_t* mask;  // n_tiles x 32
+  uint32_t* mask;  // n_tiles x 32, or null: classes only
   unsigned long long* claim;  // zeroed tile counter (warps claim tiles one at a time)
   unsigned long long* counters;  // [culled tiles, masked pairs, tiles left unclassified]
 };
@@ -310,6 +310,7 @@ struct WaveShape {
   bool trace64_nodes_smem, trace32_nodes_smem;
   int n_nodes_smem;
   int gen_bps, trace_bps;  // blocks per SM of the generation / traversal grids (0 = occupancy limit)
+  int occ_grid;            // > 0: the occlusion kernels, blocks of the list kernel
 };
 
 size_t gen_smem_bytes(bool mixed, int pmax, bool occ);
@@ -319,6 +320,64 @@ size_t trace_smem_bytes(bool fp32, int n_nodes_smem);
 cudaError_t launch_gen(const WaveShape& sh, const GenBatch* g, int sm_count, cudaStream_t st);
 cudaError_t launch_trace(const WaveShape& sh, const TraceBatch* t, bool fp32, int sm_count, cudaStream_t st);
 cudaError_t launch_resolve(const WaveShape& sh, const ResolveBatch* r, int sm_count, cudaStream_t st);
+// The listed tiles of surface meshes with occlusion (kernels_occ.cu): one
+// request's arguments, a queued pair with its list (entries pool[off, off + n):
+// leaf node << 8 | mask of the leaf's triangles; n = -1: its rays walk the
+// tree), and the launch block of one chunk.
+struct OccArgs {
+  int64_t N, nT, tile0;
+  int pmax;
+  bool mixed, lists;
+  const double* tab;
+  const float* tabf;
+  const int8_t* np;
+  const double *area, *nrm, *cen, *diam, *rad;
+  const uint8_t* flat;
+  double near_factor, cull_margin;
+  float sat_em, delta;
+  const int32_t *group, *orig;
+  double* F;
+  const NodeD* nodes;
+  const NodeF* nodesf;
+  int n_nodes;
+  const TriD* tris;
+  const TriF* trisf;
+  const float4* sat;
+  const int32_t* frontier;
+  int n_frontier;
+  const int32_t* work;
+  const uint8_t* tcls;
+  uint32_t* tmask;  // written: the queued pairs of each row of a listed tile
+};
+struct OccSlot {
+  int32_t i, j, req, n;
+  int64_t off;
+};
+struct OccQ {
+  unsigned long long* ctr;
+  OccSlot* slots;
+  int64_t scap;
+  uint32_t* pool;
+  int64_t pool_cap;
+};
+struct OccBatch {
+  const OccArgs* reqs;
+  const PairArgs* preqs;
+  const MixedArgs* mreqs;
+  const int64_t* tile_base;
+  int n_req;
+  int64_t total_tiles;
+  int groups;      // list tasks per tile (occ_groups)
+  int pmax_max;
+  int rest_parts;  // row sets of a tile in k_occ_rest (a warp each)
+  OccQ q;
+  unsigned long long* counters;
+};
+int occ_groups(int64_t n_tiles, int sm_count);
+int occ_list_grid(int sm_count);  // resident blocks of the list kernel
+// marks (or null): events recorded after the list, rest and pair kernels
+cudaError_t launch_occ(bool mixed, int pmax, const OccBatch* b, int list_grid, int sm_count, cudaStream_t st,
+                       const cudaEvent_t* marks);
 // Pair lists of the chunk's pending pairs (3-D triangles with occlusion).
 cudaError_t launch_plist(const TraceBatch* t, int sm_count, cudaStream_t st);
 // Tile classes and masks of one request (before its first chunk).

@@ -42,6 +42,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "device_hull.cuh"
 #include "device_lists.cuh"
 #include "kernels.h"
 
@@ -51,131 +52,6 @@ namespace {
 
 constexpr int kCullWarps = 4;
 
-// Pair masks: the capsule test over all 16 axes (1) or the pair lists' 4 (0).
-#ifndef RVF_MASK_FULL_AXES
-#define RVF_MASK_FULL_AXES 0
-#endif
-
-// Position of the n-th (from 0) set bit of m (n < popc(m)): binary search
-// over halves by population count.
-__device__ __forceinline__ int nth_set_bit(uint32_t m, int n) {
-  int pos = 0;
-#pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const int c = __popc(m & ((1u << s) - 1u));
-    if (n >= c) {
-      n -= c;
-      m >>= s;
-      pos += s;
-    }
-  }
-  return pos;
-}
-
-// H = conv(B_1 u B_2) of two boxes (FP32 centres c and half extents h).
-struct HullF {
-  float c[2][3], h[2][3];
-  float d[3];  // c[1] - c[0]
-};
-
-// Projection interval of the hull on w.
-__device__ __forceinline__ void hull_proj(const HullF& H, float wx, float wy, float wz, float& lo, float& hi) {
-  const float aw0 = fabsf(wx), aw1 = fabsf(wy), aw2 = fabsf(wz);
-  const float m0 = fmaf(H.c[0][0], wx, fmaf(H.c[0][1], wy, H.c[0][2] * wz));
-  const float r0 = fmaf(H.h[0][0], aw0, fmaf(H.h[0][1], aw1, H.h[0][2] * aw2));
-  const float m1 = fmaf(H.c[1][0], wx, fmaf(H.c[1][1], wy, H.c[1][2] * wz));
-  const float r1 = fmaf(H.h[1][0], aw0, fmaf(H.h[1][1], aw1, H.h[1][2] * aw2));
-  lo = fminf(m0 - r0, m1 - r1);
-  hi = fmaxf(m0 + r0, m1 + r1);
-}
-
-// True when the interval [qlo, qhi] lies farther than m |w| from the hull
-// along w (squares avoid the square root; m > 0).
-__device__ __forceinline__ bool hull_gap(const HullF& H, float wx, float wy, float wz, float qlo, float qhi,
-                                         float m) {
-  float lo, hi;
-  hull_proj(H, wx, wy, wz, lo, hi);
-  const float gap = fmaxf(qlo - hi, lo - qhi);
-  return gap > 0.0f && gap * gap > m * m * fmaf(wx, wx, fmaf(wy, wy, wz * wz));
-}
-
-// True when every point of the box lies farther than m from the hull.
-__device__ __forceinline__ bool hull_misses_box(const HullF& H, const NodeF& nd, float m) {
-  // coordinate axes
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float lo = fminf(H.c[0][k] - H.h[0][k], H.c[1][k] - H.h[1][k]);
-    const float hi = fmaxf(H.c[0][k] + H.h[0][k], H.c[1][k] + H.h[1][k]);
-    if (nd.lo[k] - hi > m || lo - nd.hi[k] > m) return true;
-  }
-  // the centroid direction crossed with each coordinate axis
-  const float bc[3] = {0.5f * (nd.lo[0] + nd.hi[0]), 0.5f * (nd.lo[1] + nd.hi[1]), 0.5f * (nd.lo[2] + nd.hi[2])};
-  const float bh[3] = {0.5f * (nd.hi[0] - nd.lo[0]), 0.5f * (nd.hi[1] - nd.lo[1]), 0.5f * (nd.hi[2] - nd.lo[2])};
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float w[3] = {0.f, 0.f, 0.f};  // d x e_k
-    w[(k + 1) % 3] = H.d[(k + 2) % 3];
-    w[(k + 2) % 3] = -H.d[(k + 1) % 3];
-    const float bm = fmaf(bc[0], w[0], fmaf(bc[1], w[1], bc[2] * w[2]));
-    const float br = fmaf(bh[0], fabsf(w[0]), fmaf(bh[1], fabsf(w[1]), bh[2] * fabsf(w[2])));
-    if (hull_gap(H, w[0], w[1], w[2], bm - br, bm + br, m)) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tri_proj(const float4& p0, const float4& p1, const float4& p2, float wx, float wy,
-                                         float wz, float& lo, float& hi) {
-  const float q0 = fmaf(p0.x, wx, fmaf(p0.y, wy, p0.z * wz));
-  const float q1 = fmaf(p1.x, wx, fmaf(p1.y, wy, p1.z * wz));
-  const float q2 = fmaf(p2.x, wx, fmaf(p2.y, wy, p2.z * wz));
-  lo = fminf(q0, fminf(q1, q2));
-  hi = fmaxf(q0, fmaxf(q1, q2));
-}
-
-// True when the triangle lies farther than m from the hull.
-__device__ __forceinline__ bool hull_misses_tri(const HullF& H, const float4& p0, const float4& p1, const float4& p2,
-                                                float m) {
-  float lo, hi;
-  // coordinate axes
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float w[3] = {k == 0 ? 1.f : 0.f, k == 1 ? 1.f : 0.f, k == 2 ? 1.f : 0.f};
-    tri_proj(p0, p1, p2, w[0], w[1], w[2], lo, hi);
-    if (hull_gap(H, w[0], w[1], w[2], lo, hi, m)) return true;
-  }
-  const float e[3][3] = {{p1.x - p0.x, p1.y - p0.y, p1.z - p0.z},
-                         {p2.x - p0.x, p2.y - p0.y, p2.z - p0.z},
-                         {p2.x - p1.x, p2.y - p1.y, p2.z - p1.z}};
-  // the normal
-  {
-    const float nx = e[0][1] * e[1][2] - e[0][2] * e[1][1];
-    const float ny = e[0][2] * e[1][0] - e[0][0] * e[1][2];
-    const float nz = e[0][0] * e[1][1] - e[0][1] * e[1][0];
-    tri_proj(p0, p1, p2, nx, ny, nz, lo, hi);
-    if (hull_gap(H, nx, ny, nz, lo, hi, m)) return true;
-  }
-  // the edges crossed with the centroid direction and with the coordinate axes
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const float* f = e[a];
-    {
-      const float* d = H.d;
-      const float wx = d[1] * f[2] - d[2] * f[1], wy = d[2] * f[0] - d[0] * f[2], wz = d[0] * f[1] - d[1] * f[0];
-      tri_proj(p0, p1, p2, wx, wy, wz, lo, hi);
-      if (hull_gap(H, wx, wy, wz, lo, hi, m)) return true;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      float w[3] = {0.f, 0.f, 0.f};  // e_k x f
-      w[(k + 1) % 3] = -f[(k + 2) % 3];
-      w[(k + 2) % 3] = f[(k + 1) % 3];
-      tri_proj(p0, p1, p2, w[0], w[1], w[2], lo, hi);
-      if (hull_gap(H, w[0], w[1], w[2], lo, hi, m)) return true;
-    }
-  }
-  return false;
-}
-
 }  // namespace
 
 // One warp per tile, grid-stride over the tiles of one request.
@@ -183,14 +59,18 @@ __device__ __forceinline__ bool hull_misses_tri(const HullF& H, const float4& p0
 #ifndef RVF_CULL_MIN_BLOCKS
 #define RVF_CULL_MIN_BLOCKS 1
 #endif
+// MASK: with step 3.  Without it (quadrature solves, whose occlusion kernel
+// builds every pair's list itself, kernels_occ.cu) a tile is decided by its
+// first surviving triangle.
+template <bool MASK>
 __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_class(const TileClassArgs a) {
   __shared__ int s_front[kCullWarps][2 * kTileFront];
   __shared__ int s_leaf[kCullWarps][kTileLeaves];
-  __shared__ int s_list[kCullWarps][kTileTris];
-  __shared__ int s_rleaf[kCullWarps][kTileLeaves];  // runs of the list: leaf node
-  __shared__ int s_rspan[kCullWarps][kTileLeaves];  //   first list entry * 16 + count
-  __shared__ int s_row[kCullWarps][kTileLeaves];    // a row's runs
-  __shared__ float s_cap[kCullWarps][32][12];        // a row's pairs: capsule start, end, direction, R, group
+  __shared__ int s_list[kCullWarps][MASK ? kTileTris : 1];
+  __shared__ int s_rleaf[kCullWarps][MASK ? kTileLeaves : 1];  // runs of the list: leaf node
+  __shared__ int s_rspan[kCullWarps][MASK ? kTileLeaves : 1];  //   first list entry * 16 + count
+  __shared__ int s_row[kCullWarps][MASK ? kTileLeaves : 1];    // a row's runs
+  __shared__ float s_cap[kCullWarps][32][12];  // a row's pairs: capsule start, end, direction, R, group
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* front = s_front[warp];
   int* leaves = s_leaf[warp];
@@ -227,7 +107,25 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
     }
     // near-field and nearly coincident pairs (lane = j, loop over the row block)
     bool near = false, tiny = false;
-    const bool classify_near = a.near_factor >= 0.0 || a.tiny_gap >= 0.0;  // mixed precision only
+    bool classify_near = a.near_factor >= 0.0 || a.tiny_gap >= 0.0;  // mixed precision only
+    HullF H;              // the tile's hull
+    double rmax = 0.0, rj_max = 0.0;
+    if (classify_near || (a.occ && a.dim3)) tile_hull(oki, okj, ci, cj, ri, rj, H, rmax, rj_max);
+    if (classify_near) {
+      // no pair of blocks whose centroid boxes lie farther apart than both
+      // thresholds (2^-20 of the coordinates allows for the boxes' FP32 rounding)
+      float dm = (float)fmax(di, dj), g2 = 0.0f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dm = fmaxf(dm, __shfl_xor_sync(kFull, dm, o));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float s = H.h[0][c] + H.h[1][c];
+        const float g = fabsf(H.d[c]) - s - 9.5367431640625e-07f * (fabsf(H.c[0][c]) + fabsf(H.c[1][c]) + s);
+        if (g > 0.0f) g2 = fmaf(g, g, g2);
+      }
+      const float lim = 1.00001f * fmaxf(dm * (float)fmax(a.near_factor, 0.0), (float)(2.0 * rmax + fmax(a.tiny_gap, 0.0)));
+      classify_near = !(g2 > lim * lim);
+    }
     for (int li = 0; li < (classify_near ? kTile : 0); ++li) {
       const double x0 = __shfl_sync(kFull, ci[0], li), x1 = __shfl_sync(kFull, ci[1], li),
                    x2 = __shfl_sync(kFull, ci[2], li);
@@ -249,49 +147,14 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
     bool all_ones = false;  // occlusion the tile cannot classify: every pair keeps its rays
     int nl = 0;             // listed triangles
     int nrun = 0;           // leaves with listed triangles (runs of the list)
-    HullF H;                // the tile's hull (occlusion, 3-D)
     float rmaxJ = 0.0f;     // largest point radius of the column block
     if (a.occ && !a.dim3) {
       all_ones = true;
     } else if (a.occ) {
-      // the hull: centroid boxes of the two blocks, rounded outwards to FP32
-      double lo[2][3], hi[2][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        lo[0][c] = oki ? ci[c] : INFINITY;
-        hi[0][c] = oki ? ci[c] : -INFINITY;
-        lo[1][c] = okj ? cj[c] : INFINITY;
-        hi[1][c] = okj ? cj[c] : -INFINITY;
-      }
-      double rmax = fmax(ri, rj);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            lo[b][c] = fmin(lo[b][c], __shfl_xor_sync(kFull, lo[b][c], o));
-            hi[b][c] = fmax(hi[b][c], __shfl_xor_sync(kFull, hi[b][c], o));
-          }
-        rmax = fmax(rmax, __shfl_xor_sync(kFull, rmax, o));
-      }
+      rmaxJ = __double2float_ru(rj_max);
       // one group per block: its triangles are skipped by every ray of the tile
       const int32_t gi0 = __shfl_sync(kFull, gi, 0), gj0 = __shfl_sync(kFull, gj, 0);
       const bool g_same = a.skip_groups && __all_sync(kFull, (!oki || gi == gi0) && (!okj || gj == gj0));
-      double rj_max = rj;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) rj_max = fmax(rj_max, __shfl_xor_sync(kFull, rj_max, o));
-      rmaxJ = __double2float_ru(rj_max);
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float l = __double2float_rd(lo[b][c]), h = __double2float_ru(hi[b][c]);
-          H.c[b][c] = 0.5f * (l + h);
-          H.h[b][c] = 0.5f * (h - l);
-        }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) H.d[c] = H.c[1][c] - H.c[0][c];
       const float Rt = __double2float_ru(rmax + a.cull_margin);
       const float mbox = Rt + a.sat_em;
       // breadth-first walk from the start frontier
@@ -347,6 +210,11 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
           }
         }
         const uint32_t m = __ballot_sync(kFull, keep);
+        if constexpr (!MASK) {
+          nl = __popc(m);
+          if (nl > 0) break;
+          continue;
+        }
         const int pos = nl + __popc(m & lanemask_lt());
         if (keep && pos < kTileTris) list[pos] = u;
         // one run per leaf of this round that kept triangles
@@ -371,7 +239,11 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
       __syncwarp();
       all_ones = over;
     }
-    if (all_ones) {
+    if constexpr (!MASK) {
+      if (all_ones || nl > 0) cls |= kClsSlow;
+      else if (a.occ) ++n_culled;
+      n_over += all_ones && lane == 0 ? 1 : 0;
+    } else if (all_ones) {
       cls |= kClsSlow;
       a.mask[t * kTile + lane] = 0xffffffffu;
       n_masked += 32;
@@ -472,10 +344,8 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
             const float4 p0 = a.sat[3 * u], p1 = a.sat[3 * u + 1], p2 = a.sat[3 * u + 2];
             const int32_t g = __float_as_int(p1.w);
             if (a.skip_groups && (g == g_i || g == __float_as_int(q[10]))) continue;
-            const float qa[3] = {q[0], q[1], q[2]}, qb[3] = {q[3], q[4], q[5]}, qd[3] = {q[6], q[7], q[8]};
-            const bool miss = RVF_MASK_FULL_AXES ? pair_misses_tri_full(qa, qb, qd, q[9], a.sat_em, p0, p1, p2)
-                                                 : pair_misses_tri(qa, qb, qd, q[9], a.sat_em, p0, p1, p2);
-            if (!miss) h |= 1u << p;
+            const float qa[3] = {q[0], q[1], q[2]}, qd[3] = {q[6], q[7], q[8]};
+            if (!pair_misses_tri(qa, qd, q[9], a.sat_em, p0, p1, p2)) h |= 1u << p;
           }
           hit |= __reduce_or_sync(kFull, h);
         }
@@ -505,16 +375,18 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
 
 cudaError_t launch_tile_class(const TileClassArgs& a, int sm_count, cudaStream_t st) {
   if (a.n_tiles <= 0) return cudaSuccess;
-  int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile_class, kCullWarps * 32, 0) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  const int64_t want = (a.n_tiles + kCullWarps - 1) / kCullWarps;
-  const int grid = (int)std::min<int64_t>(want, (int64_t)sm_count * per_sm);
-  const cudaError_t e = cudaMemsetAsync(a.claim, 0, sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
-  k_tile_class<<<(unsigned)grid, kCullWarps * 32, 0, st>>>(a);
-  return cudaGetLastError();
+  auto launch = [&](auto fn) -> cudaError_t {
+    int per_sm = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kCullWarps * 32, 0) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    const int64_t want = (a.n_tiles + kCullWarps - 1) / kCullWarps;
+    const int grid = (int)std::min<int64_t>(want, (int64_t)sm_count * per_sm);
+    const cudaError_t e = cudaMemsetAsync(a.claim, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    fn<<<(unsigned)grid, kCullWarps * 32, 0, st>>>(a);
+    return cudaGetLastError();
+  };
+  return a.mask ? launch(k_tile_class<true>) : launch(k_tile_class<false>);
 }
 
 }  // namespace rvf

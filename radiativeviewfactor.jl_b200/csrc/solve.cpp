@@ -395,7 +395,7 @@ int rvf_session_destroy(rvf_session* s) try {
     s->fast_ctr.free_();
     s->wq_ctr.free_(); s->wq_rec64.free_(); s->wq_rec32.free_(); s->wq_slots.free_(); s->wq_vis.free_(); s->wq_plist.free_(); s->wq_pool.free_();
     for (rvf::DevBuf* b : {&s->wl_pair, &s->wl_mixed, &s->wl_trace, &s->wl_resolve, &s->wl_tilebase, &s->wl_gen,
-                           &s->wl_tb, &s->wl_rb})
+                           &s->wl_tb, &s->wl_rb, &s->wl_occ, &s->wl_ob})
       b->free_();
     for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
     s->graphs.clear();

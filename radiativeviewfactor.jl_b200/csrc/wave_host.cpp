@@ -77,6 +77,36 @@ int ensure_wave(Session* s, bool two_queues, bool occ, bool lists, int pmax, int
   return 0;
 }
 
+// The occlusion kernels' pair queue and list pool, kept by the session: a slot
+// per pair of the offered tiles, up to 2^25, and eight entries per slot, halved
+// until they fit half of the budget left (chunks then hold fewer tiles); the
+// list kernel's blocks may each add one tile's 1,024 pairs beyond a full queue.
+static int ensure_occ(Session* s, int64_t n_tiles, OccQ& q, int& grid) {
+  constexpr int64_t kPool = 8;
+  int rc = 0;
+  if (!s->wq_ctr.ptr && (rc = s->wq_ctr.alloc(s, sizeof(unsigned long long) * kCtrCount))) return rc;
+  const int64_t per = (int64_t)kTile * kTile;
+  const int64_t floor = 8 * per;
+  int64_t slots = std::min<int64_t>((n_tiles + occ_list_grid(s->sm_count)) * per, (int64_t)1 << 25);
+  if (s->wq_slots.bytes < sizeof(OccSlot) * slots || s->wq_pool.bytes < sizeof(uint32_t) * kPool * slots) {
+    s->wq_slots.free_();
+    s->wq_pool.free_();
+    const size_t left = s->budget > s->used ? s->budget - s->used : 0;
+    while (slots > floor && (size_t)slots * (sizeof(OccSlot) + sizeof(uint32_t) * kPool) > left / 2)
+      slots = std::max<int64_t>(floor, slots / 2);
+    if ((rc = s->wq_slots.alloc(s, sizeof(OccSlot) * slots))) return rc;
+    if ((rc = s->wq_pool.alloc(s, sizeof(uint32_t) * kPool * slots))) return rc;
+  }
+  q = OccQ{};
+  q.ctr = s->wq_ctr.as<unsigned long long>();
+  q.slots = s->wq_slots.as<OccSlot>();
+  q.scap = (int64_t)(s->wq_slots.bytes / sizeof(OccSlot));
+  q.pool = s->wq_pool.as<uint32_t>();
+  q.pool_cap = (int64_t)(s->wq_pool.bytes / sizeof(uint32_t));
+  grid = (int)std::max<int64_t>(1, std::min<int64_t>(occ_list_grid(s->sm_count), q.scap / (2 * per)));
+  return 0;
+}
+
 int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8_t* ray_log, WaveReq& w,
                  int64_t* n_kernels) {
   const int64_t N = m->N;
@@ -89,6 +119,12 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   if (o->fault_inject & RVF_FAULT_CLAIM) w.claim_retries = 0;
   w.fast_qb = o->fast_points;
   w.fast_groups = o->fast_row_groups;  // 0: by the tile count (wave_fast)
+  // Surface meshes with occlusion run the occlusion kernels; the queue pipeline
+  // keeps ray logs (every ray's decision in a record), solves without tile
+  // classes, curve meshes and obstructions beyond the lists' 24-bit leaf and
+  // 25-bit triangle indices.
+  w.occ_lists = occ && w.dim3 && !o->disable_tile_cull && !ray_log && !(o->fault_inject & RVF_FAULT_CLAIM) &&
+            m->frontier.ptr && m->n_nodes < (1 << 24) && m->n_obs < (1 << 25);
   PairArgs& a = w.pa;
   a.N = N;
   a.nT = (N + kTile - 1) / kTile;
@@ -168,7 +204,7 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
       c.sat_em = m->sat_em;
     }
     c.cls = T->tcls.as<uint8_t>();
-    c.mask = T->tmask.as<uint32_t>();
+    c.mask = w.occ_lists ? nullptr : T->tmask.as<uint32_t>();
     if (!s->fast_ctr.ptr && (rc = s->fast_ctr.alloc(s, 256))) return rc;
     c.claim = s->fast_ctr.as<unsigned long long>() + 1;
     c.counters = s->counters.as<unsigned long long>() + 13;
@@ -176,9 +212,9 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
     if (e != cudaSuccess) return cuda_err(e, "tile classification launch");
     if (n_kernels) *n_kernels += 1;
     a.tcls = c.cls;
-    a.tmask = c.mask;
+    a.tmask = T->tmask.as<uint32_t>();
     w.ma.tcls = c.cls;
-    w.ma.tmask = c.mask;
+    w.ma.tmask = a.tmask;
     if (!ray_log) {
       // The chunked pipeline's tiles: those with ray work (or near-field /
       // nearly coincident pairs in mixed precision), in row-major order; the
@@ -214,7 +250,9 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   TraceArgs& ta = w.ta;
   ta.N = N; ta.pmax = a.pmax; ta.dim3 = a.dim3; ta.tab = a.tab; ta.tabf = w.ma.tabf; ta.cen = a.cen;
   ta.group = a.group; ta.orig = a.orig; ta.nodes = a.nodes; ta.nodesf = occ ? m->nodesf.as<NodeF>() : nullptr; ta.n_nodes = a.n_nodes;
-  ta.tris = a.tris; ta.trisf = w.ma.trisf; ta.segs = a.segs; ta.delta = w.ma.delta;
+  ta.tris = a.tris; ta.segs = a.segs;
+  ta.trisf = (occ && w.dim3) ? (o->geometric_soup ? m->trisf_geo.as<TriF>() : m->trisf_ref.as<TriF>()) : nullptr;
+  ta.delta = (float)std::ldexp(m->extent, -20);
   ta.leaf_of = (occ && w.dim3 && !o->disable_pair_lists) ? m->leaf_of.as<int32_t>() : nullptr;
   ta.sat = (occ && w.dim3) ? (o->geometric_soup ? m->sat_geo.as<float4>() : m->sat_ref.as<float4>()) : nullptr;
   ta.sat_em = m->sat_em;
@@ -223,6 +261,16 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   ta.rad = a.rad;
   ta.cull_margin = a.cull_margin;
   ta.ray_log = a.ray_log; ta.log_pm = a.log_pm;
+  if (w.occ_lists) {
+    OccArgs& x = w.oa;
+    x.N = N; x.nT = a.nT; x.pmax = a.pmax; x.mixed = w.mixed; x.lists = !o->disable_pair_lists;
+    x.tab = a.tab; x.tabf = w.ma.tabf; x.np = a.np; x.area = a.area; x.nrm = a.nrm; x.cen = a.cen;
+    x.diam = T->diam.as<double>(); x.rad = a.rad; x.flat = a.flat; x.near_factor = o->near_field_factor;
+    x.cull_margin = a.cull_margin; x.sat_em = m->sat_em; x.delta = ta.delta; x.group = a.group; x.orig = a.orig;
+    x.F = a.F; x.nodes = a.nodes; x.nodesf = ta.nodesf; x.n_nodes = a.n_nodes; x.tris = a.tris; x.trisf = ta.trisf;
+    x.sat = ta.sat; x.frontier = ta.frontier; x.n_frontier = ta.n_frontier; x.work = a.work; x.tcls = a.tcls;
+    x.tmask = T->tmask.as<uint32_t>();
+  }
   ResolveArgs& ra = w.ra;
   ra.N = N; ra.pmax = a.pmax; ra.dim3 = a.dim3; ra.tab = a.tab; ra.tabf = w.ma.tabf; ra.cen = a.cen;
   ra.diam = T->diam.as<double>(); ra.near_factor = o->near_field_factor; ra.area = a.area; ra.orig = a.orig;
@@ -265,7 +313,7 @@ WaveShape wave_shape(Session* s, WaveReq* const* reqs, int n) {
   sh.dim3 = reqs[0]->dim3;
   sh.occ = reqs[0]->occ;
   for (int r = 0; r < n; ++r) sh.pmax_max = std::max(sh.pmax_max, reqs[r]->pmax);
-  if (n == 1 && sh.occ) {
+  if (n == 1 && sh.occ && !reqs[0]->occ_lists) {
     sh.n_nodes_smem = reqs[0]->pa.n_nodes;
     sh.trace64_nodes_smem = trace_smem_bytes(false, sh.n_nodes_smem) <= (size_t)72 * 1024;
     sh.trace32_nodes_smem = sh.mixed && trace_smem_bytes(true, sh.n_nodes_smem) <= (size_t)80 * 1024;
@@ -287,6 +335,8 @@ int ensure_blocks(Session* s) {
     if ((rc = s->wl_gen.alloc(s, sizeof(GenBatch)))) return rc;
     if ((rc = s->wl_tb.alloc(s, sizeof(TraceBatch)))) return rc;
     if ((rc = s->wl_rb.alloc(s, sizeof(ResolveBatch)))) return rc;
+    if ((rc = s->wl_occ.alloc(s, sizeof(OccArgs) * kMaxBatch))) return rc;
+    if ((rc = s->wl_ob.alloc(s, sizeof(OccBatch)))) return rc;
   }
   if (!s->h_ctr) {
     const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&s->h_ctr), sizeof(unsigned long long) * kCtrCount, 0);
@@ -299,7 +349,7 @@ uint64_t shape_key(const WaveShape& sh) {
   return (uint64_t)sh.mixed | ((uint64_t)sh.dim3 << 1) | ((uint64_t)sh.occ << 2) |
          ((uint64_t)sh.trace64_nodes_smem << 4) | ((uint64_t)sh.trace32_nodes_smem << 5) |
          ((uint64_t)sh.pmax_max << 8) | ((uint64_t)sh.gen_bps << 16) | ((uint64_t)sh.trace_bps << 20) |
-         ((uint64_t)sh.n_nodes_smem << 24);
+         ((uint64_t)(sh.n_nodes_smem & 0xffffff) << 24) | ((uint64_t)sh.occ_grid << 48);
 }
 
 // The chunk's device work: counters reset, generation, traversal(s), resolve
@@ -310,6 +360,12 @@ cudaError_t enqueue_chunk(Session* s, const WaveShape& sh, bool events) {
   cudaError_t e = cudaMemsetAsync(s->wq_ctr.ptr, 0, sizeof(unsigned long long) * kCtrCount, st);
   if (e != cudaSuccess) return e;
   if (events) cudaEventRecord(s->ev[0], st);
+  if (sh.occ_grid > 0) {
+    if ((e = launch_occ(sh.mixed, sh.pmax_max, s->wl_ob.as<OccBatch>(), sh.occ_grid, s->sm_count, st,
+                        events ? &s->ev[1] : nullptr)) != cudaSuccess)
+      return e;
+    return cudaMemcpyAsync(s->h_ctr, s->wq_ctr.ptr, sizeof(unsigned long long) * kCtrCount, cudaMemcpyDeviceToHost, st);
+  }
   if ((e = launch_gen(sh, s->wl_gen.as<GenBatch>(), s->sm_count, st)) != cudaSuccess) return e;
   if (events) cudaEventRecord(s->ev[1], st);
   if (sh.occ) {
@@ -347,7 +403,8 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   double left = pp_budget > 0 ? pp_budget : 1e300;
   for (int r = 0; r < n_in && left > 0; ++r) {
     const int64_t rem = reqs_in[r]->n_tiles - reqs_in[r]->claimed;
-    if (rem <= 0) continue;
+    // one launch holds requests of one kernel: those of the oldest one's
+    if (rem <= 0 || (!reqs.empty() && reqs_in[r]->occ_lists != reqs[0]->occ_lists)) continue;
     const double per = (double)kTile * kTile * reqs_in[r]->pmax * reqs_in[r]->pmax;
     const int64_t take = (left >= per * (double)rem) ? rem : std::max<int64_t>(1, (int64_t)std::ceil(left / per));
     reqs.push_back(reqs_in[r]);
@@ -357,21 +414,31 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   if (reqs.empty()) return RVF_OK;
   const int n = (int)reqs.size();
   WaveShape sh = wave_shape(s, reqs.data(), n);
-  sh.gen_bps = gen_bps;
-  sh.trace_bps = trace_bps;
+  const bool fused = reqs[0]->occ_lists;
+  sh.gen_bps = fused ? 0 : gen_bps;
+  sh.trace_bps = fused ? 0 : trace_bps;
   std::vector<int64_t> base(n + 1, 0);
   for (int r = 0; r < n; ++r) base[r + 1] = base[r] + offer[r];
+  const bool queues = sh.occ && !fused;
   WaveQ q{};
-  if ((rc = ensure_wave(s, sh.mixed && sh.occ, sh.occ, sh.occ && sh.dim3, sh.pmax_max, base[n], q))) return rc;
+  OccBatch ob{};
+  if (fused) {
+    if ((rc = ensure_occ(s, base[n], ob.q, sh.occ_grid))) return rc;
+  } else if ((rc = ensure_wave(s, sh.mixed && queues, queues, queues && sh.dim3, sh.pmax_max, base[n], q))) {
+    return rc;
+  }
   std::vector<PairArgs> pa(n);
   std::vector<MixedArgs> ma(n);
   std::vector<TraceArgs> ta(n);
   std::vector<ResolveArgs> ra(n);
+  std::vector<OccArgs> oa(n);
   for (int r = 0; r < n; ++r) {
     pa[r] = reqs[r]->pa;
     ma[r] = reqs[r]->ma;
     ta[r] = reqs[r]->ta;
     ra[r] = reqs[r]->ra;
+    oa[r] = reqs[r]->oa;
+    oa[r].tile0 = reqs[r]->claimed;
     pa[r].tile0 = ma[r].tile0 = reqs[r]->claimed;
     pa[r].q = ma[r].q = ta[r].q = q;
   }
@@ -401,6 +468,20 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   rb.reqs = s->wl_resolve.as<ResolveArgs>();
   rb.n_req = n;
   rb.q = q;
+  if (fused) {
+    ob.reqs = s->wl_occ.as<OccArgs>();
+    ob.preqs = g.reqs;
+    ob.mreqs = g.mreqs;
+    ob.tile_base = g.tile_base;
+    ob.n_req = n;
+    ob.pmax_max = sh.pmax_max;
+    ob.total_tiles = base[n];
+    // a tile is split into tasks only when the queue holds every tile at once
+    const bool all = (base[n] + sh.occ_grid) * kTile * kTile <= ob.q.scap;
+    ob.groups = all ? occ_groups(base[n], s->sm_count) : 1;
+    ob.rest_parts = base[n] * 8 >= (int64_t)64 * s->sm_count ? 8 : 32;
+    ob.counters = g.counters;
+  }
   cudaStream_t st = s->stream;
   cudaError_t e = cudaSuccess;
   auto up = [&](DevBuf& d, const void* h, size_t bytes) {
@@ -408,12 +489,17 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   };
   up(s->wl_pair, pa.data(), sizeof(PairArgs) * n);
   up(s->wl_mixed, ma.data(), sizeof(MixedArgs) * n);
-  up(s->wl_trace, ta.data(), sizeof(TraceArgs) * n);
-  up(s->wl_resolve, ra.data(), sizeof(ResolveArgs) * n);
   up(s->wl_tilebase, base.data(), sizeof(int64_t) * (n + 1));
-  up(s->wl_gen, &g, sizeof g);
-  up(s->wl_tb, &tb, sizeof tb);
-  up(s->wl_rb, &rb, sizeof rb);
+  if (fused) {
+    up(s->wl_occ, oa.data(), sizeof(OccArgs) * n);
+    up(s->wl_ob, &ob, sizeof ob);
+  } else {
+    up(s->wl_trace, ta.data(), sizeof(TraceArgs) * n);
+    up(s->wl_resolve, ra.data(), sizeof(ResolveArgs) * n);
+    up(s->wl_gen, &g, sizeof g);
+    up(s->wl_tb, &tb, sizeof tb);
+    up(s->wl_rb, &rb, sizeof rb);
+  }
   if (e != cudaSuccess) return cuda_err(e, "launch block upload");
   bool replayed = false;
   if (use_graph) {
@@ -442,12 +528,21 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   if (info) {
     *info = ChunkInfo{};
     info->graph = replayed;
-    info->kernels = 1 + (sh.occ ? (sh.mixed ? 3 : 2) + (sh.dim3 ? 1 : 0) : 0);
+    info->kernels = (fused ? 3 : 1) + (queues ? (sh.mixed ? 3 : 2) + (sh.dim3 ? 1 : 0) : 0);
     if (!replayed) {
       float t = 0.f;
       cudaEventElapsedTime(&t, s->ev[0], s->ev[1]);
-      info->ms_gen = t;
-      if (sh.occ) {
+      if (fused) {
+        float tr = 0.f, tp = 0.f;
+        cudaEventElapsedTime(&tr, s->ev[1], s->ev[2]);
+        cudaEventElapsedTime(&tp, s->ev[2], s->ev[3]);
+        info->ms_gen = tr;
+        info->ms_trace = t + tp;
+        info->ms_lists = t;
+      } else {
+        info->ms_gen = t;
+      }
+      if (queues) {
         float t12 = 0.f, t23 = 0.f, t34 = 0.f;
         cudaEventElapsedTime(&t12, s->ev[1], s->ev[2]);
         cudaEventElapsedTime(&t23, s->ev[2], s->ev[3]);
@@ -462,10 +557,10 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
         }
       }
     }
-    info->rays_traced = (int64_t)(sh.mixed ? s->h_ctr[kCtrRec32] : s->h_ctr[kCtrRec64]);
+    info->rays_traced = (int64_t)(sh.mixed && !fused ? s->h_ctr[kCtrRec32] : s->h_ctr[kCtrRec64]);
   }
   // tiles are claimed in launch order: request r got min(claimed - base[r], its remaining tiles)
-  const int64_t got = (int64_t)s->h_ctr[kCtrTile];
+  const int64_t got = (int64_t)s->h_ctr[kCtrTile] / (fused ? ob.groups : 1);
   for (int r = 0; r < n; ++r) {
     const int64_t take = std::max<int64_t>(0, std::min<int64_t>(got - base[r], base[r + 1] - base[r]));
     reqs[r]->claimed += take;
