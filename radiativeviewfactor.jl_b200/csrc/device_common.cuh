@@ -143,15 +143,50 @@ __device__ __forceinline__ void eval_line(const double* __restrict__ coords, con
 // ---------------------------------------------------------------------------
 // view-factor kernel
 // ---------------------------------------------------------------------------
-// Reference formula (src/GPUKernels.jl:204-215 / src/ViewFactorKernel.jl:169-180),
-// bit for bit.  dim3: cos*cos/(pi r^2); otherwise cos*cos/(2 r).
+// a / b for several a with one b: y = RN(1 / b) (one division), q0 = RN(a y),
+// and twice q <- RN(q + RN(a - q b) y).  The first step leaves q0 (off by at
+// most 2 ulp) faithful, after which the second gives RN(a / b) (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990: a faithful quotient corrected once by the correctly rounded reciprocal
+// is correctly rounded).  The residuals are exact unless a is so small that
+// they underflow: such a (and b out of the middle range) take the division.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = fma(fma(-q0, b, a), y, q0);
+  return fma(fma(-q1, b, a), y, q1);
+}
+// whether a / b may be taken by div_by: a zero or 2^-700 <= |a| < 2^700 (hi words)
+__device__ __forceinline__ bool div_by_ok(double a) {
+  const unsigned h = (unsigned)(__double2hiint(a) & 0x7fffffff);
+  return h - 0x14300000u < 0x57800000u || a == 0.0;
+}
+
+// The reference's cosines (src/GPUKernels.jl:204-215 /
+// src/ViewFactorKernel.jl:169-180) and distance, bit for bit.
+__device__ __forceinline__ void reference_cosines(double rx, double ry, double rz, double r2, const double* ni,
+                                                  const double* nj, double& ci, double& cj, double& r) {
+  r = sqrt(r2);
+  double hx, hy, hz;
+  if (div_by_ok(rx) && div_by_ok(ry) && div_by_ok(rz) && div_by_ok(r)) {
+    const double y = 1.0 / r;
+    hx = div_by(rx, r, y);
+    hy = div_by(ry, r, y);
+    hz = div_by(rz, r, y);
+  } else {
+    hx = rx / r;
+    hy = ry / r;
+    hz = rz / r;
+  }
+  ci = (ni[0] * hx + ni[1] * hy) + ni[2] * hz;
+  cj = (nj[0] * (-hx) + nj[1] * (-hy)) + nj[2] * (-hz);
+}
+
+// The reference's kernel, bit for bit.  dim3: cos*cos/(pi r^2); otherwise cos*cos/(2 r).
 template <bool DIM3>
 __device__ __forceinline__ double k_reference_inl(double rx, double ry, double rz, double r2, const double* ni,
                                                   const double* nj) {
-  double r = sqrt(r2);
-  double hx = rx / r, hy = ry / r, hz = rz / r;
-  double ci = (ni[0] * hx + ni[1] * hy) + ni[2] * hz;
-  double cj = (nj[0] * (-hx) + nj[1] * (-hy)) + nj[2] * (-hz);
+  double ci, cj, r;
+  reference_cosines(rx, ry, rz, r2, ni, nj, ci, cj, r);
   if (ci <= 0.0 || cj <= 0.0) return 0.0;
   return DIM3 ? (ci * cj) / (kPiD * r2) : (ci * cj) / (2.0 * r);
 }

@@ -61,9 +61,185 @@ __device__ __forceinline__ int find_req(const int64_t* tile_base, int n_req, int
 // bit what the ray pipeline gives for pairs whose rays are all visible.
 // Out of line: their registers are allocated apart from the ray pipeline's.
 // ---------------------------------------------------------------------------
+// FP64 arithmetic.  Per point pair the FP64 pipe runs r (3), r^2 (3), the two
+// cosines' numerators (6), their product, r^4, the reciprocal (two steps) and
+// the two multiply-adds into the sum: 19 instructions, 36 before, when r^2 was
+// formed as the shadow rays form it, the reciprocal took two Newton steps and
+// signs and grazing were compared on the FP64 pipe; 1 / pi is applied once per
+// pair.  Signs and the grazing test read the high words as integers.  Bound by
+// the FP64 pipe (about half of its cycles) and instruction issue.  Measured, one
+// solve, before -> now: cylinder of 3,072 Quad8, nquad 5 (curved) 13.6 -> 8.6 ms;
+// 800 Quad4, nquad 4 (a quarter of the point pairs graze) 0.53 -> 0.39 ms; the
+// closed cube of 43,200 Tri3 (all plane) 163 -> 91 ms with its masked tiles' rest.
+//
+// 1 / x from rcp.approx.ftz.f64 (operand and result cut to 20 mantissa bits:
+// relative error e0 below 2^-18.9): with e = 1 - x y, 1 / x = y (1 + e + e^2 + ...),
+// cut after e^2 (e^3 < 2^-56).  x^-3/2 from rsqrt.approx.ftz.f64 likewise, with
+// e = 1 - x y^2: y^3 (1 + 3/2 e + 15/8 e^2 + 35/16 e^3).
+__device__ __forceinline__ double recip_scaled(double k, double x) {  // k / x
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0), k0 = k * y;
+  return fma(k0, fma(e, e, e), k0);
+}
+__device__ __forceinline__ double recip32_scaled(double k, double x) {  // k x^-3/2
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double s = y * y, e = fma(-x, s, 1.0), k0 = k * (y * s);
+  return fma(k0, e * fma(fma(2.1875, e, 1.875), e, 1.5), k0);
+}
+
+// s += w k when the sign bit of `both` is clear (di >= 0 and dj < 0), as one predicated instruction.
+__device__ __forceinline__ void fma_if_facing(double& s, double w, double k, int both) {
+  asm("{\n .reg .pred f;\n setp.ge.s32 f, %3, 0;\n @f fma.rn.f64 %0, %1, %2, %0;\n}" : "+d"(s) : "d"(w), "d"(k), "r"(both));
+}
+
+// Pairs of plane elements (one normal each) that are at least eight of their
+// sizes apart: the cosine at a point depends on that point alone --
+// n_i.(x_q - x_p) is the same for every p, up to the rounding of the element's
+// points -- so a point pair costs r, r^2, 1 / r^4 and one multiply-add, 11
+// FP64 instructions instead of 19, and no sign or grazing test.  A pair with a
+// |cos| below 1e-3 (d^2 <= limit for some d; limit = 1e-6 of the largest
+// possible r^2) is left to the general loop: its cosines would lose more than
+// three digits to the points' rounding.
+struct FlatSum {
+  double sum;  // pi times the pair's sum
+  uint32_t cast;
+  bool done;
+};
+template <int QB>
+__device__ __noinline__ FlatSum flat_fp64_q(const double* S, const double* jb, int pm, int npi, int npj,
+                                            double limit) {
+  double ni[3], nj[3], xi0[3], xj0[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    xi0[c] = S[c];
+    ni[c] = S[4 + c];
+    xj0[c] = npj > 0 ? jb[c * pm * kTile] : 0.0;
+    nj[c] = npj > 0 ? jb[(3 + c) * pm * kTile] : 0.0;
+  }
+  const int qmax = __reduce_max_sync(kFull, npj);
+  double acc = 0.0;
+  int pos_i = 0, pos_j = 0;
+  bool ok = npj > 0;
+  for (int q0 = 0; q0 < qmax; q0 += QB) {
+    double x[QB][3], inner[QB];
+#pragma unroll
+    for (int u = 0; u < QB; ++u) {
+      const int q = q0 + u < npj ? q0 + u : 0;  // past the element's points: the first again, not summed
+#pragma unroll
+      for (int c = 0; c < 3; ++c) x[u][c] = npj > 0 ? jb[(c * pm + q) * kTile] : 1.0;
+      inner[u] = 0.0;
+    }
+    for (int p = 0; p < npi; ++p) {
+      const double2 s0 = *reinterpret_cast<const double2*>(S + 8 * p), s1 = *reinterpret_cast<const double2*>(S + 8 * p + 2);
+      const double x0 = s0.x, x1 = s0.y, x2 = s1.x;
+      const double dj = fma(nj[0], x0 - xj0[0], fma(nj[1], x1 - xj0[1], nj[2] * (x2 - xj0[2])));
+      const bool facing = __double2hiint(dj) >= 0;
+      const double w = facing ? s1.y * dj : 0.0;
+      if (q0 == 0) {
+        ok = ok && dj * dj > limit;
+        pos_j += facing ? 1 : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < QB; ++u) {
+        const double rx = x[u][0] - x0, ry = x[u][1] - x1, rz = x[u][2] - x2;
+        const double r2 = fma(rx, rx, fma(ry, ry, rz * rz)), r4 = r2 * r2;
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r4));
+        const double e = fma(-r4, y, 1.0);
+        inner[u] = fma(w, fma(y, fma(e, e, e), y), inner[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < QB; ++u) {
+      if (q0 + u < npj) {
+        const double di = fma(ni[0], x[u][0] - xi0[0], fma(ni[1], x[u][1] - xi0[1], ni[2] * (x[u][2] - xi0[2])));
+        ok = ok && di * di > limit;
+        if (__double2hiint(di) >= 0) {
+          acc = fma(jb[(6 * pm + q0 + u) * kTile] * di, inner[u], acc);
+          ++pos_i;
+        }
+      }
+    }
+  }
+  return FlatSum{acc, (uint32_t)(pos_i * pos_j), ok};
+}
+// The point block by the rule's size: no or few idle points (7: 7, 13 and 49
+// points; 5: 5 and 25; 3: 3 and 9; 4: 4, 16, 36, 64, and the others).
+__device__ __forceinline__ FlatSum flat_fp64(const double* S, const double* jb, int pm, int npi, int npj,
+                                             double limit) {
+  if (pm == 7 || pm == 13 || pm == 49) return flat_fp64_q<7>(S, jb, pm, npi, npj, limit);
+  if (pm == 5 || pm == 25) return flat_fp64_q<5>(S, jb, pm, npi, npj, limit);
+  if (pm == 3 || pm == 9) return flat_fp64_q<3>(S, jb, pm, npi, npj, limit);
+  return flat_fp64_q<4>(S, jb, pm, npi, npj, limit);
+}
+
+// shared memory of a block's eight staged rows
+__host__ __device__ __forceinline__ size_t stage_bytes(int pmax) { return (size_t)8 * 8 * pmax * sizeof(double); }
+
+// The source element's points for the warp's loops: eight doubles a point (x, y,
+// z, w, n) in shared memory, read by broadcast 16-byte loads from one address,
+// where the table's component-major layout costs a load and an address per value.
+__device__ __forceinline__ void stage_row(const double* ib, double* S, int pm) {
+  const int lane = threadIdx.x & 31;
+  const float per = 1.0f / (float)pm;  // v + 1/2 is at least 1/128 from a multiple of pm, v < 448
+  __syncwarp();                        // the previous row's readers
+  for (int v = lane; v < kComp * pm; v += 32) {
+    const int c = (int)(((float)v + 0.5f) * per), p = v - c * pm;
+    S[8 * p + (c < 3 ? c : c == 6 ? 3 : c + 1)] = ib[v * kTile];
+  }
+  __syncwarp();
+}
+
+// One column (point q of the lane's element, all points p of the source) with
+// k_fast's arithmetic, which takes the reference formula at grazing point pairs.
+struct ColumnSum {
+  double inner;  // scaled as the fast loop's
+  uint32_t cast;
+};
+template <bool DIM3>
+__device__ __noinline__ ColumnSum column_exact(const double* ib, const double* jq, int pm, int npi) {
+  ColumnSum s{0.0, 0};
+  double xj[3], nj[3];
+  for (int c = 0; c < 3; ++c) {
+    xj[c] = jq[c * pm * kTile];
+    nj[c] = jq[(3 + c) * pm * kTile];
+  }
+#pragma unroll 2
+  for (int p = 0; p < npi; ++p) {
+    double xi[3], ni[3];
+    for (int c = 0; c < 3; ++c) {
+      xi[c] = ib[(c * pm + p) * kTile];
+      ni[c] = ib[((3 + c) * pm + p) * kTile];
+    }
+    const double rx = xj[0] - xi[0], ry = xj[1] - xi[1], rz = xj[2] - xi[2];
+    const double r2 = (rx * rx + ry * ry) + rz * rz;
+    // k_fast's tests; the reference's cosines where one grazes (their product over
+    // r^2 needs no correctly rounded quotient)
+    double k = 0.0;  // pi K (3-D), 2 K (2-D)
+    if (!(r2 < 1e-30)) {
+      const double di = fma(ni[0], rx, fma(ni[1], ry, ni[2] * rz));
+      const double dj = -fma(nj[0], rx, fma(nj[1], ry, nj[2] * rz));
+      const double thr = 1e-10 * r2;
+      if (di * di <= thr || dj * dj <= thr) {
+        double ci, cj, r;
+        reference_cosines(rx, ry, rz, r2, ni, nj, ci, cj, r);
+        if (ci > 0.0 && cj > 0.0) k = recip_scaled(ci * cj, DIM3 ? r2 : r);
+      } else if (di > 0.0 && dj > 0.0) {
+        k = DIM3 ? recip_scaled(di * dj, r2 * r2) : recip32_scaled(di * dj, r2);
+      }
+    }
+    s.cast += k > 0.0 ? 1 : 0;
+    s.inner = fma(ib[(6 * pm + p) * kTile], -k, s.inner);
+  }
+  return s;
+}
+
 template <bool DIM3, bool OCC, int QB>
-__device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const double* iblk, int64_t bi, int64_t bj,
-                                                   int li0, int lane, uint32_t& n_pp, uint32_t& n_rays, uint32_t skip = 0) {
+__device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const double* iblk, double* S, int64_t bi,
+                                                   int64_t bj, int li0, int lane, uint32_t& n_pp, uint32_t& n_rays,
+                                                   uint32_t skip = 0) {
   const int64_t N = a.N;
   const int pm = a.pmax;
   const int64_t j = bj * kTile + lane;
@@ -84,100 +260,95 @@ __device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const doub
     if (valid && a.flat[i] && a.flat[j] && a.nrm[3 * i] == a.nrm[3 * j] && a.nrm[3 * i + 1] == a.nrm[3 * j + 1] &&
         a.nrm[3 * i + 2] == a.nrm[3 * j + 2])
       npj = 0;
-    const int qmax = __reduce_max_sync(kFull, npj);
+    // every distance of the pair's points lies within s of |c_j - c_i|
+    double d2 = 0.0, s2 = 0.0;
+    if (npj > 0) {
+      const double dx = a.cen[3 * j] - a.cen[3 * i], dy = a.cen[3 * j + 1] - a.cen[3 * i + 1],
+                   dz = a.cen[3 * j + 2] - a.cen[3 * i + 2];
+      const double s = a.rad[i] + a.rad[j];
+      d2 = dx * dx + dy * dy + dz * dz;
+      s2 = s * s;
+    }
     const double* ib = iblk + li;
-    double acc = 0.0;
+    stage_row(ib, S, pm);
+    double acc = 0.0;  // minus pi (3-D) or 2 (2-D) times the pair's sum
+    n_pp += (uint32_t)(npi * npj);
+    if constexpr (DIM3) {
+      const int npf = npj > 0 && a.flat[i] && a.flat[j] && d2 > 64.0 * s2 ? npj : 0;
+      if (__any_sync(kFull, npf > 0)) {
+        const FlatSum f = flat_fp64(S, jb, pm, npi, npf, 1.27e-6 * d2);
+        if (f.done) {
+          acc = -f.sum;
+          if (OCC) n_rays += f.cast;
+          npj = 0;
+        }
+      }
+    }
+    // points of the pair may nearly coincide: every column with k_fast's own arithmetic
+    const bool tiny = !(d2 > 1.0001 * s2 + 1e-28);
+    // no |cos| is below 1e-5 when every |d| exceeds 1e-5 of the largest distance
+    // (hi words, so the threshold is rounded up by one)
+    const int graze = __double2hiint(1e-5 * sqrt(2.0 * (d2 + s2))) + 1;
+    const int qmax = __reduce_max_sync(kFull, npj);
     for (int q0 = 0; q0 < qmax; q0 += QB) {
-      double xq[QB][3], nq[QB][3], wq[QB];
+      double xq[QB][3], nq[QB][3];
 #pragma unroll
       for (int u = 0; u < QB; ++u) {
-        const int q = q0 + u;
-        const bool lq = q < npj;
+        // past the element's points: the first one again (finite, not summed)
+        const int q = q0 + u < npj ? q0 + u : 0;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          xq[u][c] = lq ? jb[(c * pm + q) * kTile] : 0.0;
-          nq[u][c] = lq ? jb[((3 + c) * pm + q) * kTile] : 0.0;
+          xq[u][c] = jok ? jb[(c * pm + q) * kTile] : 0.0;
+          nq[u][c] = jok ? jb[((3 + c) * pm + q) * kTile] : 0.0;
         }
-        wq[u] = lq ? jb[(6 * pm + q) * kTile] : 0.0;
       }
       double inner[QB];
+      int least[QB];      // smallest hi|d| of the column
+      uint32_t cast[QB];
 #pragma unroll
-      for (int u = 0; u < QB; ++u) inner[u] = 0.0;
-      // k_fast with its grazing branch taken out of the loop: a lane that
-      // meets a grazing point pair (either |cos| within 1e-5 of zero) forms
-      // the chunk again below with k_fast's own arithmetic
-      bool graze = false;
-      uint32_t cast = 0;
-      const int ulim = npj - q0;
+      for (int u = 0; u < QB; ++u) {
+        inner[u] = 0.0;
+        least[u] = 0x7fffffff;
+        cast[u] = 0;
+      }
       for (int p = 0; p < npi; ++p) {
-        double xi[3], ni[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          xi[c] = ib[(c * pm + p) * kTile];
-          ni[c] = ib[((3 + c) * pm + p) * kTile];
-        }
-        const double wi = ib[(6 * pm + p) * kTile];
-        // straight-line over the block: a point q0 + u >= npj has zero
-        // normal and weight, so its dj is -0 and its K zero (it only must not
-        // ask for the grazing redo)
+        const double2* s = reinterpret_cast<const double2*>(S + 8 * p);
+        const double2 s0 = s[0], s1 = s[1], s2v = s[2];
+        const double xi[3] = {s0.x, s0.y, s1.x}, ni[3] = {s2v.x, s2v.y, S[8 * p + 6]};
+        const double wi = s1.y;
 #pragma unroll
         for (int u = 0; u < QB; ++u) {
           const double rx = xq[u][0] - xi[0], ry = xq[u][1] - xi[1], rz = xq[u][2] - xi[2];
-          const double r2 = (rx * rx + ry * ry) + rz * rz;
+          const double r2 = fma(rx, rx, fma(ry, ry, rz * rz));
           const double di = fma(ni[0], rx, fma(ni[1], ry, ni[2] * rz));
-          const double dj = -fma(nq[u][0], rx, fma(nq[u][1], ry, nq[u][2] * rz));
-          const double thr = 1e-10 * r2;
-          const bool big = !(r2 < 1e-30);
-          graze = graze || (u < ulim && big && (di * di <= thr || dj * dj <= thr));
-          double K = 0.0;
-          if (big && di > 0.0 && dj > 0.0)
-            K = DIM3 ? (di * dj) * rcp_nr(kPiD * (r2 * r2)) : (di * dj) * rcp_nr(2.0 * (r2 * sqrt(r2)));
-          cast += K > 0.0 ? 1 : 0;
-          inner[u] = fma(wi, K, inner[u]);
+          const double dj = fma(nq[u][0], rx, fma(nq[u][1], ry, nq[u][2] * rz));  // minus the reference's
+          const int hi = __double2hiint(di), hj = __double2hiint(dj), both = hi | ~hj;
+          least[u] = min(least[u], min(hi & 0x7fffffff, hj & 0x7fffffff));
+          const double K = DIM3 ? recip_scaled(di * dj, r2 * r2) : recip32_scaled(di * dj, r2);
+          fma_if_facing(inner[u], wi, K, both);
+          if (OCC) cast[u] += (uint32_t)~both >> 31;
         }
       }
-      if (__any_sync(kFull, graze) && graze) {  // rare: the chunk again, exactly as the ray pipeline forms it
-        cast = 0;
 #pragma unroll
-        for (int u = 0; u < QB; ++u) inner[u] = 0.0;
-        for (int p = 0; p < npi; ++p) {
-          double xi[3], ni[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            xi[c] = ib[(c * pm + p) * kTile];
-            ni[c] = ib[((3 + c) * pm + p) * kTile];
-          }
-          const double wi = ib[(6 * pm + p) * kTile];
-#pragma unroll
-          for (int u = 0; u < QB; ++u) {
-            if (q0 + u < npj) {
-              const double rx = xq[u][0] - xi[0], ry = xq[u][1] - xi[1], rz = xq[u][2] - xi[2];
-              const double r2 = (rx * rx + ry * ry) + rz * rz;
-              // k_fast, with the reference formula in line
-              double K = 0.0;
-              if (!(r2 < 1e-30)) {
-                const double di = fma(ni[0], rx, fma(ni[1], ry, ni[2] * rz));
-                const double dj = -fma(nq[u][0], rx, fma(nq[u][1], ry, nq[u][2] * rz));
-                const double thr = 1e-10 * r2;
-                if (di * di <= thr || dj * dj <= thr) K = k_reference_inl<DIM3>(rx, ry, rz, r2, ni, nq[u]);
-                else if (di > 0.0 && dj > 0.0)
-                  K = DIM3 ? (di * dj) * rcp_nr(kPiD * (r2 * r2)) : (di * dj) * rcp_nr(2.0 * (r2 * sqrt(r2)));
-              }
-              cast += K > 0.0 ? 1 : 0;
-              inner[u] = fma(wi, K, inner[u]);
-            }
-          }
+      for (int u = 0; u < QB; ++u) {
+        // a column with a grazing point pair (a |cos| within 1e-5 of zero, where
+        // the sign of the fast form could differ from the reference's) again
+        const bool again = q0 + u < npj && (tiny || least[u] <= graze);
+        if (__any_sync(kFull, again) && again) {
+          const ColumnSum c = column_exact<DIM3>(ib, jb + (q0 + u) * kTile, pm, npi);
+          inner[u] = c.inner;
+          cast[u] = c.cast;
+        }
+        if (q0 + u < npj) {
+          acc = fma(jb[(6 * pm + q0 + u) * kTile], inner[u], acc);
+          if (OCC) n_rays += cast[u];
         }
       }
-      if (OCC) n_rays += cast;
-#pragma unroll
-      for (int u = 0; u < QB; ++u)
-        if (q0 + u < npj) acc = fma(wq[u], inner[u], acc);
     }
-    n_pp += (uint32_t)(npi * npj);
     if (valid) {
-      a.F[oi + oj * N] = acc / a.area[i];
-      a.F[oj + oi * N] = acc / a.area[j];
+      const double raw = acc * (DIM3 ? -1.0 / kPiD : -0.5);
+      a.F[oi + oj * N] = raw / a.area[i];
+      a.F[oj + oi * N] = raw / a.area[j];
     } else if (j == i) {
       a.F[oi + oi * N] = 0.0 / a.area[i];
     }
@@ -271,26 +442,26 @@ __device__ __forceinline__ void gen_fast_mixed_body(const MixedArgs& a, const fl
 // Out of line inside the chunked generation kernels, whose own registers are
 // allocated for the ray pipeline.
 template <bool DIM3, bool OCC, int QB>
-__device__ __noinline__ void gen_fast_fp64(const PairArgs& a, const double* iblk, int64_t bi, int64_t bj, int li0, int lane, uint32_t& n_pp,
-    uint32_t& n_rays, uint32_t skip = 0) {
-  gen_fast_fp64_body<DIM3, OCC, QB>(a, iblk, bi, bj, li0, lane, n_pp, n_rays, skip);
+__device__ __noinline__ void gen_fast_fp64(const PairArgs& a, const double* iblk, double* S, int64_t bi, int64_t bj,
+                                           int li0, int lane, uint32_t& n_pp, uint32_t& n_rays, uint32_t skip) {
+  gen_fast_fp64_body<DIM3, OCC, QB>(a, iblk, S, bi, bj, li0, lane, n_pp, n_rays, skip);
 }
 template <bool OCC, int QB>
-__device__ __noinline__ void gen_fast_mixed(const MixedArgs& a, const float* iblk, int64_t bi, int64_t bj, int li0, int lane, uint32_t& n_pp,
-    uint32_t& n_rays, uint32_t skip = 0) {
+__device__ __noinline__ void gen_fast_mixed(const MixedArgs& a, const float* iblk, int64_t bi, int64_t bj, int li0,
+                                            int lane, uint32_t& n_pp, uint32_t& n_rays, uint32_t skip) {
   gen_fast_mixed_body<OCC, QB>(a, iblk, bi, bj, li0, lane, n_pp, n_rays, skip);
 }
 
 // The fast loop with the point block for the rule's size (li0 as there).
 template <bool DIM3, bool OCC>
-__device__ __forceinline__ void fast_fp64(const PairArgs& a, const double* iblk, int64_t bi, int64_t bj, int li0, int lane, uint32_t& n_pp,
-    uint32_t& n_rays, uint32_t skip = 0) {
-  if (a.pmax <= 3) gen_fast_fp64<DIM3, OCC, 3>(a, iblk, bi, bj, li0, lane, n_pp, n_rays, skip);
-  else gen_fast_fp64<DIM3, OCC, 4>(a, iblk, bi, bj, li0, lane, n_pp, n_rays, skip);
+__device__ __forceinline__ void fast_fp64(const PairArgs& a, const double* iblk, double* S, int64_t bi, int64_t bj,
+                                          int li0, int lane, uint32_t& n_pp, uint32_t& n_rays, uint32_t skip = 0) {
+  if (a.pmax <= 3) gen_fast_fp64<DIM3, OCC, 3>(a, iblk, S, bi, bj, li0, lane, n_pp, n_rays, skip);
+  else gen_fast_fp64<DIM3, OCC, 4>(a, iblk, S, bi, bj, li0, lane, n_pp, n_rays, skip);
 }
 template <bool OCC>
-__device__ __forceinline__ void fast_mixed(const MixedArgs& a, const float* iblk, int64_t bi, int64_t bj, int li0, int lane, uint32_t& n_pp,
-    uint32_t& n_rays, uint32_t skip = 0) {
+__device__ __forceinline__ void fast_mixed(const MixedArgs& a, const float* iblk, int64_t bi, int64_t bj, int li0,
+                                           int lane, uint32_t& n_pp, uint32_t& n_rays, uint32_t skip = 0) {
   const int pm = a.pmax;
   if (pm == 7 || pm == 13 || pm == 49) gen_fast_mixed<OCC, 7>(a, iblk, bi, bj, li0, lane, n_pp, n_rays, skip);
   else if (pm == 5 || pm == 25) gen_fast_mixed<OCC, 5>(a, iblk, bi, bj, li0, lane, n_pp, n_rays, skip);

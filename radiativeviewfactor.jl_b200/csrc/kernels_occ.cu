@@ -632,7 +632,9 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
 // rows of a tile when there are many).
 template <bool MIXED>
 __global__ void __launch_bounds__(256, 2) k_occ_rest(const OccBatch* __restrict__ Lp) {
+  extern __shared__ __align__(128) unsigned char smem[];
   const OccBatch& B = *Lp;
+  double* S = reinterpret_cast<double*>(smem) + (threadIdx.x >> 5) * 8 * B.pmax_max;
   const int lane = threadIdx.x & 31;
   const unsigned long long claimed = *(volatile unsigned long long*)(B.q.ctr + kCtrTile) / (unsigned)B.groups;
   const int64_t n_tiles = claimed < (unsigned long long)B.total_tiles ? (int64_t)claimed : B.total_tiles;
@@ -671,7 +673,7 @@ __global__ void __launch_bounds__(256, 2) k_occ_rest(const OccBatch* __restrict_
         else row_visible_mixed(a, bi, bj, li, skip, near, cnt);
       } else {
         const PairArgs& a = B.preqs[r];
-        fast_fp64<true, true>(a, a.tab + bi * kComp * a.pmax * kTile, bi, bj, li + 8, lane, cnt[0], cnt[1], skip);
+        fast_fp64<true, true>(a, a.tab + bi * kComp * a.pmax * kTile, S, bi, bj, li + 8, lane, cnt[0], cnt[1], skip);
       }
     }
   }
@@ -1066,7 +1068,7 @@ cudaError_t launch_occ(bool mixed, int pmax, const OccBatch* b, int list_grid, i
   k_occ_list<<<(unsigned)list_grid, 256, sizeof(OccTile), st>>>(b);
   if ((e = mark(0)) != cudaSuccess) return e;
   if (mixed) k_occ_rest<true><<<(unsigned)(2 * sm_count), 256, 0, st>>>(b);
-  else k_occ_rest<false><<<(unsigned)(2 * sm_count), 256, 0, st>>>(b);
+  else k_occ_rest<false><<<(unsigned)(2 * sm_count), 256, stage_bytes(pmax), st>>>(b);
   if ((e = mark(1)) != cudaSuccess) return e;
   auto pairs = [&](auto fn, size_t smem) -> cudaError_t {
     const cudaError_t e1 = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

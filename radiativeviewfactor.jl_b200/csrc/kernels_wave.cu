@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(256, 2) k_gen_fp64(const GenBatch* __restrict_
   double* iblk = reinterpret_cast<double*>(smem);
   uint64_t* ring = reinterpret_cast<uint64_t*>(iblk + kComp * pmL * kTile) + threadIdx.x;
   uint64_t* bar = reinterpret_cast<uint64_t*>(iblk + kComp * pmL * kTile) + (OCC ? kRun * 256 : 0);
+  double* S = reinterpret_cast<double*>(bar + 2) + (threadIdx.x >> 5) * 8 * pmL;
   __shared__ int64_t s_tile;
   __shared__ int s_req;
   __shared__ unsigned long long s_used, s_slots;
@@ -268,8 +269,8 @@ __global__ void __launch_bounds__(256, 2) k_gen_fp64(const GenBatch* __restrict_
     }
     phase ^= 1u;
 
-    if (a.tcls && !(cls & kClsSlow) && !a.ray_log) {  // block-uniform: no ray of the tile can be blocked
-      if (!a.fast_done) fast_fp64<DIM3, OCC>(a, iblk, bi, bj, warp, lane, n_pp, n_rays);
+    if (!OCC || (a.tcls && !(cls & kClsSlow) && !a.ray_log)) {  // block-uniform: no ray of the tile can be blocked
+      if (!a.fast_done || !a.tcls) fast_fp64<DIM3, OCC>(a, iblk, S, bi, bj, warp, lane, n_pp, n_rays);
       __syncthreads();
       if (OCC && threadIdx.x == 0) resv_release(Q, need, need_s);
       continue;
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(256, 2) k_gen_fp64(const GenBatch* __restrict_
       const int64_t i = bi * kTile + li;
       if (i >= N) continue;  // warp-uniform
       if (a.tcls && !a.ray_log && s_mask[li] == 0u) {  // no ray of this row can be blocked
-        fast_fp64<DIM3, OCC>(a, iblk, bi, bj, li + 8, lane, n_pp, n_rays);
+        fast_fp64<DIM3, OCC>(a, iblk, S, bi, bj, li + 8, lane, n_pp, n_rays);
         continue;
       }
       const bool valid = (j < N) && (i < j);
@@ -1245,6 +1246,8 @@ __device__ __forceinline__ bool fast_task(unsigned long long* task_ctr, int64_t 
 template <bool DIM3, bool OCC, int QB>
 __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_fp64(const PairArgs a, unsigned long long* task_ctr,
                                                                        unsigned long long* counters) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  double* S = reinterpret_cast<double*>(smem) + (threadIdx.x >> 5) * 8 * a.pmax;
   const int lane = threadIdx.x & 31;
   uint32_t n_pp = 0, n_rays = 0;
   int64_t t;
@@ -1253,7 +1256,7 @@ __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_fp64(const Pa
     int64_t bi, bj;
     tile_coords(t, a.nT, bi, bj);
     const double* ib = a.tab + bi * kComp * a.pmax * kTile;
-    for (int r = r0; r < r1; ++r) gen_fast_fp64_body<DIM3, OCC, QB>(a, ib, bi, bj, r, lane, n_pp, n_rays);
+    for (int r = r0; r < r1; ++r) gen_fast_fp64_body<DIM3, OCC, QB>(a, ib, S, bi, bj, r, lane, n_pp, n_rays);
   }
   const uint64_t s_pp = warp_sum_u64(n_pp), s_rays = warp_sum_u64(n_rays);
   if (lane == 0 && counters) {
@@ -1323,8 +1326,9 @@ cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs&
                         unsigned long long* task_ctr, unsigned long long* counters, int sm_count, cudaStream_t st) {
   auto launch = [&](auto fn, const auto& args) -> cudaError_t {
     int per_sm = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
-    fn<<<(unsigned)(sm_count * per_sm), 256, 0, st>>>(args, task_ctr, counters);
+    const size_t smem = mixed ? 0 : stage_bytes(a.pmax);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    fn<<<(unsigned)(sm_count * per_sm), 256, smem, st>>>(args, task_ctr, counters);
     return cudaGetLastError();
   };
   if (mixed) {
@@ -1352,9 +1356,9 @@ cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs&
 }
 size_t gen_smem_bytes(bool mixed, int pmax, bool occ) {
   // tile block, then (occlusion) the per-warp FP64 staging (mixed) and the
-  // per-lane runs, then the mbarrier
+  // per-lane runs, then the mbarrier and (FP64) the warps' staged rows
   const size_t stage = occ ? ((mixed ? (size_t)8 * 64 + kRunMix * 256 : (size_t)kRun * 256)) * sizeof(uint64_t) : 0;
-  return gen_tab_bytes(mixed, pmax) + stage + 16;
+  return gen_tab_bytes(mixed, pmax) + stage + 16 + (mixed ? 0 : stage_bytes(pmax));
 }
 
 size_t trace_smem_bytes(bool fp32, int n_nodes_smem) {
