@@ -135,6 +135,25 @@ void DevBuf::free_() {
   owner = nullptr;
 }
 
+int PinBuf::need(size_t n) {
+  if (bytes >= n) return RVF_OK;
+  free_();
+  n += n / 4 + 4096;
+  const cudaError_t e = cudaHostAlloc(&ptr, n, cudaHostAllocDefault);
+  if (e != cudaSuccess) {
+    ptr = nullptr;
+    cudaGetLastError();
+    return set_err(RVF_ENOMEM, "cudaHostAlloc(%zu): %s", n, cudaGetErrorString(e));
+  }
+  bytes = n;
+  return RVF_OK;
+}
+void PinBuf::free_() {
+  if (ptr) cudaFreeHost(ptr);
+  ptr = nullptr;
+  bytes = 0;
+}
+
 void release_spares(Session* s, size_t need) {
   std::lock_guard<std::mutex> lk(s->spare_mu);
   // the oldest first (the front of the list), until `need` more bytes fit

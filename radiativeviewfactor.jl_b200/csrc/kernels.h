@@ -474,6 +474,7 @@ cudaError_t launch_prep(const PrepArgs& a, cudaStream_t st);
 cudaError_t launch_prep_f32(const PrepF32Args& a, cudaStream_t st);
 size_t pair_smem_bytes(int pmax, int n_nodes_smem, bool occ);
 cudaError_t launch_pairs_fp64(const PairArgs& a, int sm_count, cudaStream_t st);
+int reduce_chunks(int64_t N, int sm_count);  // column chunks of the reductions
 cudaError_t launch_reduce(const RedArgs& a, cudaStream_t st);
 
 }  // namespace rvf

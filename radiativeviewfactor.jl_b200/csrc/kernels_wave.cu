@@ -1229,7 +1229,7 @@ __device__ __forceinline__ bool fast_task(unsigned long long* task_ctr, int64_t 
     k = __shfl_sync(kFull, k, 0);
     const unsigned long long tile = k / (unsigned)groups;
     if (tile >= (unsigned long long)n_tiles) return false;
-    if (tcls[tile] & skip) continue;
+    if (tcls && (tcls[tile] & skip)) continue;
     const int g = (int)(k - tile * (unsigned)groups);
     t = (int64_t)tile;
     if (groups <= 8) {

@@ -79,6 +79,20 @@ struct FastTune {
 
 }  // namespace rvf
 
+namespace rvf {
+// a page-locked host buffer, grown on demand
+struct PinBuf {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  int need(size_t n);
+  void free_();
+  template <typename T>
+  T* as() const {
+    return static_cast<T*>(ptr);
+  }
+};
+}  // namespace rvf
+
 struct rvf_session {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -101,8 +115,12 @@ struct rvf_session {
   // device launch blocks, pinned counter readback, graphs per launch shape
   rvf::DevBuf wq_ctr, wq_rec64, wq_rec32, wq_slots, wq_vis, wq_plist, wq_pool;
   rvf::DevBuf fast_ctr;  // tile counter of the kernel for tiles without ray work
-  rvf::DevBuf wl_pair, wl_mixed, wl_trace, wl_resolve, wl_tilebase, wl_gen, wl_tb, wl_rb, wl_occ, wl_ob;
-  unsigned long long* h_ctr = nullptr;
+  rvf::DevBuf wl;  // launch blocks of a chunk (wave_host.cpp: ensure_blocks)
+  unsigned long long* h_ctr = nullptr;  // kCtrCount counters, then the error flags
+  // page-locked staging: a copy from or to pageable memory goes through the
+  // driver and blocks the caller each time
+  rvf::PinBuf h_wl, h_tiles, h_result;
+  cudaEvent_t tev[24] = {};  // time marks of one solve, read after its last synchronisation
   std::map<uint64_t, cudaGraphExec_t> graphs;
   std::set<rvf_mesh*> meshes;
   cudaEvent_t ev[8] = {};
@@ -166,6 +184,7 @@ int mesh_upload(Session* s, const rvf_mesh_desc* d, rvf_mesh** out);
 int ensure_tables(Session* s, rvf_mesh* m, int nquad, Tables** out);
 // solve.cpp helpers shared with the serving loop (callers hold s->mu)
 int read_err(Session* s);
+int err_status(int herr);  // status of the kernels' error flags
 int validate_options(const rvf_mesh* m, const rvf_options* o);
 int no_progress(Session* s);
 int reduce_alloc(Session* s, rvf_mesh* m);  // the reductions' buffers (before any kernel runs)

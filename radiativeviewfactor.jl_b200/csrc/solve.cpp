@@ -17,24 +17,33 @@ using namespace rvf;
 
 namespace {
 
-struct EvTimer {
-  cudaStream_t st;
-  cudaEvent_t a = nullptr, b = nullptr;
-  explicit EvTimer(cudaStream_t s) : st(s) {
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, st);
+// Time spans of one solve on its stream: events recorded as the work is queued
+// and read after the solve's last synchronisation (reading one at once would
+// wait for the device in the middle of the solve).
+struct Spans {
+  Session* s;
+  int used = 0;
+  struct Span {
+    int a, b;
+    double* ms;
+  } span[12];
+  int n = 0;
+  explicit Spans(Session* s_) : s(s_) {}
+  int begin(double* ms) {
+    span[n] = Span{used, -1, ms};
+    cudaEventRecord(s->tev[used++], s->stream);
+    return n++;
   }
-  double stop() {
-    cudaEventRecord(b, st);
-    cudaEventSynchronize(b);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, a, b);
-    return ms;
+  void end(int k) {
+    span[k].b = used;
+    cudaEventRecord(s->tev[used++], s->stream);
   }
-  ~EvTimer() {
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+  void read() {
+    for (int k = 0; k < n; ++k) {
+      float ms = 0.f;
+      if (span[k].b >= 0 && cudaEventElapsedTime(&ms, s->tev[span[k].a], s->tev[span[k].b]) == cudaSuccess)
+        *span[k].ms += ms;
+    }
   }
 };
 
@@ -47,6 +56,10 @@ int read_err(Session* s) {
   cudaError_t e = cudaMemcpyAsync(&herr, s->err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return cuda_err(e, "kernel execution");
+  return err_status(herr);
+}
+
+int err_status(int herr) {
   if (herr & kErrWaitTimeout) return set_err(RVF_ETIMEDOUT, "a bounded device wait gave up (shared-memory copy did not complete)");
   if (herr & kErrBadInput) return set_err(RVF_EINVAL, "kernel reported invalid input");
   return RVF_OK;
@@ -194,7 +207,7 @@ cudaError_t launch_self_pairs(Session* s, const PairArgs& pa, cudaStream_t st) {
 int reduce_alloc(Session* s, rvf_mesh* m) {
   const int64_t N = m->N;
   if (N == 0 || m->G == 0) return RVF_OK;
-  const int n_chunks = (int)std::min<int64_t>(256, std::max<int64_t>(1, (1 << 20) / std::max<int64_t>(N, 1)));
+  const int n_chunks = reduce_chunks(N, s->sm_count);
   int rc;
   if (m->part.bytes < sizeof(double) * n_chunks * m->G * N)
     if ((rc = m->part.alloc(s, sizeof(double) * n_chunks * m->G * N))) return rc;
@@ -212,7 +225,7 @@ int reduce_alloc(Session* s, rvf_mesh* m) {
 int run_reduce(Session* s, rvf_mesh* m, const double* area) {
   const int64_t N = m->N;
   if (N == 0 || m->G == 0) return RVF_OK;
-  const int n_chunks = (int)std::min<int64_t>(256, std::max<int64_t>(1, (1 << 20) / std::max<int64_t>(N, 1)));
+  const int n_chunks = reduce_chunks(N, s->sm_count);
   int rc = reduce_alloc(s, m);
   if (rc) return rc;
   RedArgs r{};
@@ -368,6 +381,8 @@ int rvf_session_create(const rvf_session_opts* opts, rvf_session** out) try {
     return cuda_err(e, "cudaStreamCreate");
   for (cudaEvent_t& v : s->ev)
     if ((e = cudaEventCreate(&v)) != cudaSuccess) return cuda_err(e, "cudaEventCreate");
+  for (cudaEvent_t& v : s->tev)
+    if ((e = cudaEventCreate(&v)) != cudaSuccess) return cuda_err(e, "cudaEventCreate");
   size_t fr = 0, tot = 0;
   cudaMemGetInfo(&fr, &tot);
   s->budget = (opts && opts->hbm_budget_bytes) ? opts->hbm_budget_bytes : (size_t)(0.9 * (double)fr);
@@ -394,15 +409,16 @@ int rvf_session_destroy(rvf_session* s) try {
     s->counters.free_();
     s->fast_ctr.free_();
     s->wq_ctr.free_(); s->wq_rec64.free_(); s->wq_rec32.free_(); s->wq_slots.free_(); s->wq_vis.free_(); s->wq_plist.free_(); s->wq_pool.free_();
-    for (rvf::DevBuf* b : {&s->wl_pair, &s->wl_mixed, &s->wl_trace, &s->wl_resolve, &s->wl_tilebase, &s->wl_gen,
-                           &s->wl_tb, &s->wl_rb, &s->wl_occ, &s->wl_ob})
-      b->free_();
+    s->wl.free_();
+    for (rvf::PinBuf* b : {&s->h_wl, &s->h_tiles, &s->h_result}) b->free_();
     for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
     s->graphs.clear();
     rvf::release_spares(s);
     if (s->h_ctr) cudaFreeHost(s->h_ctr);
     s->h_ctr = nullptr;
     for (cudaEvent_t v : s->ev)
+      if (v) cudaEventDestroy(v);
+    for (cudaEvent_t v : s->tev)
       if (v) cudaEventDestroy(v);
     cudaStreamDestroy(s->stream);
     if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
@@ -538,17 +554,18 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
   if (mixed && !(o->near_field_factor >= 0.0)) return set_err(RVF_EINVAL, "near_field_factor must be >= 0");
   rvf_stats S{};
   int64_t n_kernels = 0;  // kernels of this library launched by this call
-  EvTimer total(s->stream);
+  Spans spans(s);
+  const int sp_total = spans.begin(&S.ms_total);
   const int64_t N = m->N;
   Tables* T = nullptr;
   const double* area_res = nullptr;  // element areas of this result, caller's order
   if (!mc) {
-    EvTimer t(s->stream);
+    const int t = spans.begin(&S.ms_prep);
     const bool fresh = m->tables.find(o->nquad) == m->tables.end();
     if ((rc = ensure_tables(s, m, o->nquad, &T))) return rc;
     if ((rc = reduce_alloc(s, m))) return rc;
     if (fresh && N > 0) n_kernels += 1;
-    S.ms_prep = t.stop();
+    spans.end(t);
     area_res = T->area_orig.as<double>();
   } else {
     if (m->mc_area.bytes < sizeof(double) * std::max<int64_t>(N, 1))
@@ -577,19 +594,18 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
   }
   if (mc) {  // src/GPUMCKernels.jl:295-328
     {
-      EvTimer tc(s->stream);
+      const int t = spans.begin(&S.ms_cull);
       if ((rc = mc_classify(s, m, o))) return rc;
-      S.ms_cull = tc.stop();
+      spans.end(t);
     }
     McArgs c{};
     fill_mc_args(s, m, o, o->ray_log ? log.as<uint8_t>() : nullptr, c);
     if (N > 0) {
-      EvTimer t(s->stream);
+      const int t = spans.begin(&S.ms_pairs);
       cudaError_t e = launch_mc(c, s->sm_count, s->stream);
       if (e != cudaSuccess) return cuda_err(e, "Monte Carlo kernel launch");
       n_kernels += 2;
-      S.ms_pairs = t.stop();
-      if ((rc = read_err(s))) return rc;
+      spans.end(t);
     }
   } else {
   if (N > 0) {
@@ -599,14 +615,14 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
     cudaError_t e = cudaSuccess;
     WaveReq w;
     {
-      EvTimer tc(s->stream);
+      const int t = spans.begin(&S.ms_cull);
       if ((rc = wave_prepare(s, m, T, o, o->ray_log ? log.as<uint8_t>() : nullptr, w, &n_kernels))) return rc;
-      S.ms_cull = tc.stop();
+      spans.end(t);
     }
     {
-      EvTimer tf(s->stream);
+      const int t = spans.begin(&S.ms_gen);
       if ((rc = wave_fast(s, w, &n_kernels))) return rc;
-      S.ms_gen += tf.stop();
+      spans.end(t);
     }
     // Duffy and self pairs overwrite F after the pipeline: no early columns then
     if (F_elem && N > 1 && !(o->use_duffy && m->dim == 2) && !o->self_vf) {
@@ -622,7 +638,7 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
           (e = cudaStreamWaitEvent(s->copy_stream, s->ev[7], 0)) != cudaSuccess)
         return cuda_err(e, "download ordering");
     }
-    EvTimer t(s->stream);
+    const int t = spans.begin(&S.ms_pairs);
     WaveReq* one = &w;
     // the columns finished by earlier chunks are queued for download while
     // the next chunk runs
@@ -645,7 +661,7 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
       dl_upto = before;
       if ((rc = wave_chunk(s, &one, 1, false, &ci, 0, 0, pp_budget, &queue_columns))) return rc;
       if (dl_err != cudaSuccess) return cuda_err(dl_err, "F column download");
-      if ((rc = read_err(s))) return rc;
+      if ((rc = err_status((int)s->h_ctr[kCtrCount]))) return rc;
       n_kernels += ci.kernels;
       S.n_chunks += 1;
       S.ms_gen += ci.ms_gen;
@@ -661,12 +677,11 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
       if ((e = launch_self_pairs(s, w.pa, s->stream)) != cudaSuccess) return cuda_err(e, "self-pair kernel launch");
       n_kernels += 1;
     }
-    S.ms_pairs = t.stop();
-    if ((rc = read_err(s))) return rc;
+    spans.end(t);
     // Duffy integrals overwrite the singular Quad8 pairs (Duffy for
     // Quad8-Quad8 surface pairs only, src/DuffyKernel.jl:461-463)
     if (o->use_duffy && m->dim == 2) {
-      EvTimer td(s->stream);
+      const int td = spans.begin(&S.ms_duffy);
       DuffyArgs d{};
       if ((rc = ensure_duffy(s, m, o->nquad, &d.p01, &d.w01))) return rc;
       d.N = N;
@@ -685,9 +700,8 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
         if ((e = launch_duffy(d, s->stream)) != cudaSuccess) return cuda_err(e, "Duffy kernel launch");
         n_kernels += 1;
       }
-      S.ms_duffy = td.stop();
+      spans.end(td);
       S.n_duffy_pairs = m->n_duffy;
-      if ((rc = read_err(s))) return rc;
     }
     if (N == 1) {  // raw 1x1 zero, area 0 -> F = 0/0 (the reference's result for one element)
       double nanv = std::nan("");
@@ -696,38 +710,54 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
   }
   }  // quadrature
   {
-    EvTimer t(s->stream);
+    const int t = spans.begin(&S.ms_reduce);
     if ((rc = run_reduce(s, m, area_res))) return rc;
     if (N > 0 && m->G > 0) n_kernels += 3;
-    S.ms_reduce = t.stop();
+    spans.end(t);
   }
-  m->has_result = true;
-  m->result_area = area_res;
+  // everything but F comes back through page-locked memory behind one
+  // synchronisation: counters, error flags, areas, row sums, group results
+  const size_t G = (size_t)m->G, n_res = 16 + 1 + 2 * (size_t)N + G * G + G;
+  if ((rc = s->h_result.need(sizeof(double) * n_res))) return rc;
+  unsigned long long* c = s->h_result.as<unsigned long long>();
+  double* hA = s->h_result.as<double>() + 17;
+  double *hrs = hA + N, *hFg = hrs + N, *hAg = hFg + G * G;
+  const bool groups = N > 0 && m->G > 0;
   {
-    EvTimer t(s->stream);
+    const int t = spans.begin(&S.ms_download);
     cudaError_t e = cudaSuccess;
-    if (F_elem && N > 0 && !dl.host)
-      e = cudaMemcpyAsync(F_elem, m->F.ptr, sizeof(double) * N * N, cudaMemcpyDeviceToHost, s->stream);
+    auto down = [&](void* h, const void* d, size_t bytes) {
+      if (e == cudaSuccess && bytes > 0) e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s->stream);
+    };
+    if (F_elem && N > 0 && !dl.host) down(F_elem, m->F.ptr, sizeof(double) * N * N);
     if (e == cudaSuccess && dl.host) {
       e = dl.advance(w_tiles);  // every row: nothing left unless a chunk was cut short
       if (e == cudaSuccess) e = cudaStreamSynchronize(s->copy_stream);
     }
-    if (e == cudaSuccess && A_elem && N > 0) e = cudaMemcpyAsync(A_elem, area_res, sizeof(double) * N, cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess && F_group && m->G > 0 && N > 0)
-      e = cudaMemcpyAsync(F_group, m->Fgroup.ptr, sizeof(double) * m->G * m->G, cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess && A_group && m->G > 0 && N > 0)
-      e = cudaMemcpyAsync(A_group, m->Agroup.ptr, sizeof(double) * m->G, cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess && row_sums && N > 0)
-      e = cudaMemcpyAsync(row_sums, m->rowsum.ptr, sizeof(double) * N, cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess && o->ray_log)
-      e = cudaMemcpyAsync(o->ray_log, log.ptr, log_bytes, cudaMemcpyDeviceToHost, s->stream);
+    down(c, s->counters.ptr, sizeof(unsigned long long) * 16);
+    c[16] = 0;
+    down(c + 16, s->err.ptr, sizeof(int));
+    if (N > 0) down(hA, area_res, sizeof(double) * N);
+    if (groups) {
+      down(hrs, m->rowsum.ptr, sizeof(double) * N);
+      down(hFg, m->Fgroup.ptr, sizeof(double) * G * G);
+      down(hAg, m->Agroup.ptr, sizeof(double) * G);
+    }
+    if (o->ray_log) down(o->ray_log, log.ptr, log_bytes);
+    spans.end(t);
+    spans.end(sp_total);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return cuda_err(e, "device->host copy");
-    S.ms_download = t.stop();
+    if ((rc = err_status((int)(c[16] & 0xffffffffu)))) return rc;
+    m->has_result = true;
+    m->result_area = area_res;
+    if (A_elem && N > 0) std::memcpy(A_elem, hA, sizeof(double) * N);
+    if (groups && F_group) std::memcpy(F_group, hFg, sizeof(double) * G * G);
+    if (groups && A_group) std::memcpy(A_group, hAg, sizeof(double) * G);
+    if (groups && row_sums) std::memcpy(row_sums, hrs, sizeof(double) * N);
   }
   if (st) {
-    unsigned long long c[16] = {};
-    cudaMemcpy(c, s->counters.ptr, sizeof c, cudaMemcpyDeviceToHost);
+    spans.read();
     S.n_pairs = N * (N - 1) / 2;
     S.n_point_pairs = (int64_t)c[0];
     S.n_rays = (int64_t)c[1];
@@ -746,14 +776,11 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
     S.n_tiles_culled = (int64_t)c[13];
     S.n_pairs_masked = (int64_t)c[14];
     S.n_tiles_unclassified = (int64_t)c[15];
-    if (N > 0 && m->G > 0) {
-      std::vector<double> rs(N);
-      cudaMemcpy(rs.data(), m->rowsum.ptr, sizeof(double) * N, cudaMemcpyDeviceToHost);
+    if (groups) {
       double mx = 0.0;
-      for (double v : rs) mx = std::max(mx, std::fabs(v - 1.0));
+      for (int64_t i = 0; i < N; ++i) mx = std::max(mx, std::fabs(hrs[i] - 1.0));
       S.max_row_sum_dev = mx;
     }
-    S.ms_total = total.stop();
     *st = S;
   }
   return RVF_OK;

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.h"
@@ -174,7 +175,13 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   }
   // Tile classes: which pairs' shadow rays may be blocked, which tiles are
   // near field (kernels_cull.cu); recomputed by every solve.
-  if (!o->disable_tile_cull && N > 0) {
+  if (!o->disable_tile_cull && N > 0 && !occ && !w.mixed) {
+    // no rays and no near field: every tile is quadrature only
+    w.fast_all = true;
+    w.n_tiles = 0;
+    w.n_fast_tiles = a.n_tiles;
+    w.row_end.assign((size_t)a.nT, 0);
+  } else if (!o->disable_tile_cull && N > 0) {
     int rc = 0;
     const size_t nt = (size_t)a.n_tiles;
     if (T->tcls.bytes < nt && (rc = T->tcls.alloc(s, nt))) return rc;
@@ -219,31 +226,30 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
       // The chunked pipeline's tiles: those with ray work (or near-field /
       // nearly coincident pairs in mixed precision), in row-major order; the
       // others go to the quadrature-only kernel (wave_fast).
-      std::vector<uint8_t> cls(nt);
-      cudaError_t e2 = cudaMemcpyAsync(cls.data(), c.cls, nt, cudaMemcpyDeviceToHost, s->stream);
+      const size_t list_at = (nt + 255) & ~(size_t)255;
+      if ((rc = s->h_tiles.need(list_at + sizeof(int32_t) * nt))) return rc;
+      const uint8_t* cls = s->h_tiles.as<uint8_t>();
+      int32_t* work = reinterpret_cast<int32_t*>(s->h_tiles.as<uint8_t>() + list_at);
+      cudaError_t e2 = cudaMemcpyAsync(s->h_tiles.ptr, c.cls, nt, cudaMemcpyDeviceToHost, s->stream);
       if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(s->stream);
       if (e2 != cudaSuccess) return cuda_err(e2, "tile classes");
       const uint8_t need = w.mixed ? (uint8_t)(kClsSlow | kClsNear | kClsTiny) : (uint8_t)kClsSlow;
-      std::vector<int32_t> work;
       w.row_end.assign((size_t)a.nT, 0);
-      int64_t t = 0;
+      int64_t t = 0, n_work = 0;
       for (int64_t bi = 0; bi < a.nT; ++bi) {
         for (int64_t bj = bi; bj < a.nT; ++bj, ++t)
-          if (cls[(size_t)t] & need) work.push_back((int32_t)t);
-        w.row_end[(size_t)bi] = (int64_t)work.size();
+          if (cls[(size_t)t] & need) work[n_work++] = (int32_t)t;
+        w.row_end[(size_t)bi] = n_work;
       }
-      if (!work.empty()) {
-        if (T->twork.bytes < sizeof(int32_t) * work.size() &&
-            (rc = T->twork.alloc(s, sizeof(int32_t) * work.size())))
-          return rc;
-        e2 = cudaMemcpyAsync(T->twork.ptr, work.data(), sizeof(int32_t) * work.size(), cudaMemcpyHostToDevice,
-                             s->stream);
-        if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(s->stream);  // the host vector goes out of scope
+      if (n_work > 0) {
+        if (T->twork.bytes < sizeof(int32_t) * n_work && (rc = T->twork.alloc(s, sizeof(int32_t) * n_work))) return rc;
+        // (the buffer is next written after a synchronisation of this stream)
+        e2 = cudaMemcpyAsync(T->twork.ptr, work, sizeof(int32_t) * n_work, cudaMemcpyHostToDevice, s->stream);
         if (e2 != cudaSuccess) return cuda_err(e2, "tile list upload");
       }
       a.work = T->twork.as<int32_t>();
       w.ma.work = a.work;
-      w.n_tiles = (int64_t)work.size();
+      w.n_tiles = n_work;
       w.n_fast_tiles = a.n_tiles - w.n_tiles;
     }
   }
@@ -288,7 +294,7 @@ int fast_groups_auto(int64_t n_tiles, int sm_count) {
 }
 
 int wave_fast(Session* s, WaveReq& w, int64_t* n_kernels) {
-  if (!w.pa.tcls || w.pa.ray_log || w.pa.n_tiles == 0) return 0;
+  if ((!w.pa.tcls && !w.fast_all) || (w.pa.ray_log && !w.fast_all) || w.pa.n_tiles == 0) return 0;
   int rc = 0;
   if (!s->fast_ctr.ptr && (rc = s->fast_ctr.alloc(s, 256))) return rc;
   w.pa.fast_groups = w.ma.fast_groups =
@@ -324,25 +330,40 @@ WaveShape wave_shape(Session* s, WaveReq* const* reqs, int n) {
 
 namespace {
 
+// Launch blocks of a chunk: the batch structs at fixed offsets (a captured
+// graph keeps their addresses), then the requests' arguments as many as the
+// launch has; filled in page-locked memory and copied at once.
+constexpr size_t kAtGen = 0, kAtTrace = 256, kAtResolve = 512, kAtOcc = 768, kAtArgs = 1024;
+static_assert(sizeof(GenBatch) <= 256 && sizeof(TraceBatch) <= 256 && sizeof(ResolveBatch) <= 256 &&
+                  sizeof(OccBatch) <= 256,
+              "batch structs fit their places");
+constexpr size_t kBlocksBytes =
+    kAtArgs + 6 * 256 + sizeof(int64_t) * (kMaxBatch + 1) +
+    (sizeof(PairArgs) + sizeof(MixedArgs) + sizeof(TraceArgs) + sizeof(ResolveArgs) + sizeof(OccArgs)) * kMaxBatch;
+
 int ensure_blocks(Session* s) {
   int rc = 0;
-  if (!s->wl_pair.ptr) {
-    if ((rc = s->wl_pair.alloc(s, sizeof(PairArgs) * kMaxBatch))) return rc;
-    if ((rc = s->wl_mixed.alloc(s, sizeof(MixedArgs) * kMaxBatch))) return rc;
-    if ((rc = s->wl_trace.alloc(s, sizeof(TraceArgs) * kMaxBatch))) return rc;
-    if ((rc = s->wl_resolve.alloc(s, sizeof(ResolveArgs) * kMaxBatch))) return rc;
-    if ((rc = s->wl_tilebase.alloc(s, sizeof(int64_t) * (kMaxBatch + 1)))) return rc;
-    if ((rc = s->wl_gen.alloc(s, sizeof(GenBatch)))) return rc;
-    if ((rc = s->wl_tb.alloc(s, sizeof(TraceBatch)))) return rc;
-    if ((rc = s->wl_rb.alloc(s, sizeof(ResolveBatch)))) return rc;
-    if ((rc = s->wl_occ.alloc(s, sizeof(OccArgs) * kMaxBatch))) return rc;
-    if ((rc = s->wl_ob.alloc(s, sizeof(OccBatch)))) return rc;
-  }
+  if (!s->wl.ptr && (rc = s->wl.alloc(s, kBlocksBytes))) return rc;
+  if ((rc = s->h_wl.need(kBlocksBytes))) return rc;
   if (!s->h_ctr) {
-    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&s->h_ctr), sizeof(unsigned long long) * kCtrCount, 0);
+    const cudaError_t e =
+        cudaHostAlloc(reinterpret_cast<void**>(&s->h_ctr), sizeof(unsigned long long) * (kCtrCount + 1), 0);
     if (e != cudaSuccess) return cuda_err(e, "cudaHostAlloc");
   }
   return 0;
+}
+
+template <typename T>
+T* block(Session* s, size_t at) {
+  return reinterpret_cast<T*>(s->wl.as<unsigned char>() + at);
+}
+
+// the chunk's counters and error flags to the host
+cudaError_t copy_counters(Session* s) {
+  const cudaError_t e = cudaMemcpyAsync(s->h_ctr, s->wq_ctr.ptr, sizeof(unsigned long long) * kCtrCount,
+                                        cudaMemcpyDeviceToHost, s->stream);
+  if (e != cudaSuccess) return e;
+  return cudaMemcpyAsync(s->h_ctr + kCtrCount, s->err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
 }
 
 uint64_t shape_key(const WaveShape& sh) {
@@ -361,32 +382,32 @@ cudaError_t enqueue_chunk(Session* s, const WaveShape& sh, bool events) {
   if (e != cudaSuccess) return e;
   if (events) cudaEventRecord(s->ev[0], st);
   if (sh.occ_grid > 0) {
-    if ((e = launch_occ(sh.mixed, sh.pmax_max, s->wl_ob.as<OccBatch>(), sh.occ_grid, s->sm_count, st,
+    if ((e = launch_occ(sh.mixed, sh.pmax_max, block<OccBatch>(s, kAtOcc), sh.occ_grid, s->sm_count, st,
                         events ? &s->ev[1] : nullptr)) != cudaSuccess)
       return e;
-    return cudaMemcpyAsync(s->h_ctr, s->wq_ctr.ptr, sizeof(unsigned long long) * kCtrCount, cudaMemcpyDeviceToHost, st);
+    return copy_counters(s);
   }
-  if ((e = launch_gen(sh, s->wl_gen.as<GenBatch>(), s->sm_count, st)) != cudaSuccess) return e;
+  if ((e = launch_gen(sh, block<GenBatch>(s, kAtGen), s->sm_count, st)) != cudaSuccess) return e;
   if (events) cudaEventRecord(s->ev[1], st);
   if (sh.occ) {
     // the pair lists count as traversal time (the first traversal phase)
     const bool lists = sh.dim3;
     auto plist = [&]() -> cudaError_t {
       if (events) cudaEventRecord(s->ev[5], st);
-      const cudaError_t el = launch_plist(s->wl_tb.as<TraceBatch>(), s->sm_count, st);
+      const cudaError_t el = launch_plist(block<TraceBatch>(s, kAtTrace), s->sm_count, st);
       if (events) cudaEventRecord(s->ev[6], st);
       return el;
     };
     if (lists && sh.mixed && (e = plist()) != cudaSuccess) return e;
-    if (sh.mixed && (e = launch_trace(sh, s->wl_tb.as<TraceBatch>(), true, s->sm_count, st)) != cudaSuccess) return e;
+    if (sh.mixed && (e = launch_trace(sh, block<TraceBatch>(s, kAtTrace), true, s->sm_count, st)) != cudaSuccess) return e;
     if (events) cudaEventRecord(s->ev[2], st);
     if (lists && !sh.mixed && (e = plist()) != cudaSuccess) return e;
-    if ((e = launch_trace(sh, s->wl_tb.as<TraceBatch>(), false, s->sm_count, st)) != cudaSuccess) return e;
+    if ((e = launch_trace(sh, block<TraceBatch>(s, kAtTrace), false, s->sm_count, st)) != cudaSuccess) return e;
     if (events) cudaEventRecord(s->ev[3], st);
-    if ((e = launch_resolve(sh, s->wl_rb.as<ResolveBatch>(), s->sm_count, st)) != cudaSuccess) return e;
+    if ((e = launch_resolve(sh, block<ResolveBatch>(s, kAtResolve), s->sm_count, st)) != cudaSuccess) return e;
     if (events) cudaEventRecord(s->ev[4], st);
   }
-  return cudaMemcpyAsync(s->h_ctr, s->wq_ctr.ptr, sizeof(unsigned long long) * kCtrCount, cudaMemcpyDeviceToHost, st);
+  return copy_counters(s);
 }
 
 }  // namespace
@@ -427,25 +448,23 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   } else if ((rc = ensure_wave(s, sh.mixed && queues, queues, queues && sh.dim3, sh.pmax_max, base[n], q))) {
     return rc;
   }
-  std::vector<PairArgs> pa(n);
-  std::vector<MixedArgs> ma(n);
-  std::vector<TraceArgs> ta(n);
-  std::vector<ResolveArgs> ra(n);
-  std::vector<OccArgs> oa(n);
-  for (int r = 0; r < n; ++r) {
-    pa[r] = reqs[r]->pa;
-    ma[r] = reqs[r]->ma;
-    ta[r] = reqs[r]->ta;
-    ra[r] = reqs[r]->ra;
-    oa[r] = reqs[r]->oa;
-    oa[r].tile0 = reqs[r]->claimed;
-    pa[r].tile0 = ma[r].tile0 = reqs[r]->claimed;
-    pa[r].q = ma[r].q = ta[r].q = q;
-  }
+  size_t at = kAtArgs;
+  unsigned char* hw = s->h_wl.as<unsigned char>();
+  auto place = [&](auto fill, auto* kind) {  // n arguments of one kind; their device address
+    using T = std::remove_pointer_t<decltype(kind)>;
+    T* h = reinterpret_cast<T*>(hw + at);
+    for (int r = 0; r < n; ++r) fill(h[r] = T{}, *reqs[r]);
+    T* d = block<T>(s, at);
+    at = (at + sizeof(T) * n + 255) & ~(size_t)255;
+    return d;
+  };
   GenBatch g{};
-  g.reqs = s->wl_pair.as<PairArgs>();
-  g.mreqs = s->wl_mixed.as<MixedArgs>();
-  g.tile_base = s->wl_tilebase.as<int64_t>();
+  std::memcpy(hw + at, base.data(), sizeof(int64_t) * (n + 1));
+  g.tile_base = block<int64_t>(s, at);
+  at = (at + sizeof(int64_t) * (n + 1) + 255) & ~(size_t)255;
+  g.reqs = place([&](PairArgs& x, WaveReq& w) { x = w.pa; x.tile0 = w.claimed; x.q = q; }, (PairArgs*)nullptr);
+  if (sh.mixed)
+    g.mreqs = place([&](MixedArgs& x, WaveReq& w) { x = w.ma; x.tile0 = w.claimed; x.q = q; }, (MixedArgs*)nullptr);
   g.n_req = n;
   g.pmax_max = sh.pmax_max;
   g.total_tiles = base[n];
@@ -454,22 +473,8 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   g.q = q;
   g.counters = s->counters.as<unsigned long long>();
   g.err = s->err.as<int>();
-  TraceBatch tb{};
-  tb.reqs = s->wl_trace.as<TraceArgs>();
-  tb.n_req = n;
-  tb.nodes64_in_smem = sh.trace64_nodes_smem;
-  tb.nodes32_in_smem = sh.trace32_nodes_smem;
-  tb.smem_nodes64 = reqs[0]->nodes_d;
-  tb.smem_nodes32 = reqs[0]->nodes_f;
-  tb.n_nodes_smem = sh.n_nodes_smem;
-  tb.q = q;
-  tb.counters = g.counters;
-  ResolveBatch rb{};
-  rb.reqs = s->wl_resolve.as<ResolveArgs>();
-  rb.n_req = n;
-  rb.q = q;
   if (fused) {
-    ob.reqs = s->wl_occ.as<OccArgs>();
+    ob.reqs = place([&](OccArgs& x, WaveReq& w) { x = w.oa; x.tile0 = w.claimed; }, (OccArgs*)nullptr);
     ob.preqs = g.reqs;
     ob.mreqs = g.mreqs;
     ob.tile_base = g.tile_base;
@@ -481,25 +486,28 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
     ob.groups = all ? occ_groups(base[n], s->sm_count) : 1;
     ob.rest_parts = base[n] * 8 >= (int64_t)64 * s->sm_count ? 8 : 32;
     ob.counters = g.counters;
+    std::memcpy(hw + kAtOcc, &ob, sizeof ob);
+  } else {
+    TraceBatch tb{};
+    tb.reqs = place([&](TraceArgs& x, WaveReq& w) { x = w.ta; x.q = q; }, (TraceArgs*)nullptr);
+    tb.n_req = n;
+    tb.nodes64_in_smem = sh.trace64_nodes_smem;
+    tb.nodes32_in_smem = sh.trace32_nodes_smem;
+    tb.smem_nodes64 = reqs[0]->nodes_d;
+    tb.smem_nodes32 = reqs[0]->nodes_f;
+    tb.n_nodes_smem = sh.n_nodes_smem;
+    tb.q = q;
+    tb.counters = g.counters;
+    ResolveBatch rb{};
+    rb.reqs = place([&](ResolveArgs& x, WaveReq& w) { x = w.ra; }, (ResolveArgs*)nullptr);
+    rb.n_req = n;
+    rb.q = q;
+    std::memcpy(hw + kAtGen, &g, sizeof g);
+    std::memcpy(hw + kAtTrace, &tb, sizeof tb);
+    std::memcpy(hw + kAtResolve, &rb, sizeof rb);
   }
   cudaStream_t st = s->stream;
-  cudaError_t e = cudaSuccess;
-  auto up = [&](DevBuf& d, const void* h, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d.ptr, h, bytes, cudaMemcpyHostToDevice, st);
-  };
-  up(s->wl_pair, pa.data(), sizeof(PairArgs) * n);
-  up(s->wl_mixed, ma.data(), sizeof(MixedArgs) * n);
-  up(s->wl_tilebase, base.data(), sizeof(int64_t) * (n + 1));
-  if (fused) {
-    up(s->wl_occ, oa.data(), sizeof(OccArgs) * n);
-    up(s->wl_ob, &ob, sizeof ob);
-  } else {
-    up(s->wl_trace, ta.data(), sizeof(TraceArgs) * n);
-    up(s->wl_resolve, ra.data(), sizeof(ResolveArgs) * n);
-    up(s->wl_gen, &g, sizeof g);
-    up(s->wl_tb, &tb, sizeof tb);
-    up(s->wl_rb, &rb, sizeof rb);
-  }
+  cudaError_t e = cudaMemcpyAsync(s->wl.ptr, hw, at, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_err(e, "launch block upload");
   bool replayed = false;
   if (use_graph) {

@@ -19,6 +19,7 @@ struct WaveReq {
   OccArgs oa{};
   bool mixed = false, occ = false, dim3 = true;
   bool occ_lists = false;  // the listed tiles run in the occlusion kernels (kernels_occ.cu), without ray queues
+  bool fast_all = false;  // every tile is quadrature only (no classes needed)
   int pmax = 0;
   int64_t n_tiles = 0;  // tiles of the chunked pipeline (every upper-triangle tile, or the listed ones)
   std::vector<int64_t> row_end;  // with a tile list: listed tiles in tile rows 0..r (for the F download)
