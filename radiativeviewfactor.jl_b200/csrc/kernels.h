@@ -13,7 +13,8 @@ namespace rvf {
 enum : int {
   kCtrTile = 0,    // tile claims
   kCtrResv = 1,    // reserved queue records (low 38 bits) and pending-pair slots (high bits)
-  kCtrSpare = 2,
+  kCtrWalk = 2,    // occlusion kernels: queued pairs without a list
+  kCtrWalkHead = 1,  //   and their progress (kCtrResv is the queue pipeline's)
   kCtrRec64 = 3,   // records in the FP64 queue
   kCtrRec32 = 4,   // records in the FP32 queue
   kCtrSlots = 5,   // pending-pair slots in use
@@ -349,8 +350,13 @@ struct OccArgs {
   const uint8_t* tcls;
   uint32_t* tmask;  // written: the queued pairs of each row of a listed tile
 };
+enum : int {
+  kOccSame = 1 << 8,   // the elements share one normal
+  kOccNear = 1 << 9,   // near field (mixed precision)
+  kOccOut = 1 << 10,   // every ray misses the root box (mixed precision)
+};
 struct OccSlot {
-  int32_t i, j, req, n;
+  int32_t i, j, req, n;  // req: the request, with the pair's flags above its low byte
   int64_t off;
 };
 struct OccQ {

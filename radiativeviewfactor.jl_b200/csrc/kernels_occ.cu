@@ -389,7 +389,8 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
     if (threadIdx.x == 0) {
       s_tile = -1;
       // a tile needs at most 1,024 queue slots; the launch's blocks may each hold one more tile
-      const unsigned long long used = *(volatile unsigned long long*)(Q.ctr + kCtrSlots),
+      const unsigned long long used = *(volatile unsigned long long*)(Q.ctr + kCtrSlots) +
+                                      *(volatile unsigned long long*)(Q.ctr + kCtrWalk),
                                pool = *(volatile unsigned long long*)(Q.ctr + kCtrPool);
       if (used + (unsigned long long)gridDim.x * kTile * kTile <= (unsigned long long)Q.scap &&
           pool <= (unsigned long long)Q.pool_cap) {
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
       const int64_t i = bi * kTile + li;
       if (i >= N) break;
       const bool valid = okj && i < j;
-      int n = 0;  // the lane's pair: list entries, or -1 when the list does not fit
+      int n = 0;  // the lane's pair: list entries, -1: to be built by its own walk, -2: none
       if (nrun > 0) {
         const double xr[3] = {t.cen[3 * i], t.cen[3 * i + 1], t.cen[3 * i + 2]};
         const double rr = t.rad[i];
@@ -555,9 +556,7 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
       if (lane == 0) t.tmask[tile * kTile + li] = queued;
       if (queued == 0) continue;
       const bool mine = (queued >> lane) & 1u;
-      unsigned long long slot = 0, off = 0;
-      if (lane == 0) slot = atomicAdd(Q.ctr + kCtrSlots, (unsigned long long)__popc(queued));
-      slot = __shfl_sync(kFull, slot, 0) + __popc(queued & lanemask_lt());
+      unsigned long long off = 0;
       if (!t.lists && mine) n = -2;  // pair lists switched off: the rays walk the tree
       const int want = mine && n > 0 ? n : 0;
       int incl = want;
@@ -603,14 +602,33 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
           off = oo;
         }
       }
+      // list pairs from the front of the slots, the others from the back
+      const uint32_t walks = __ballot_sync(kFull, mine && n < 0), lists = queued & ~walks;
+      unsigned long long slot = 0, wslot = 0;
+      if (lane == 0 && lists) slot = atomicAdd(Q.ctr + kCtrSlots, (unsigned long long)__popc(lists));
+      if (lane == 0 && walks) wslot = atomicAdd(Q.ctr + kCtrWalk, (unsigned long long)__popc(walks));
+      slot = __shfl_sync(kFull, slot, 0) + __popc(lists & lanemask_lt());
+      wslot = __shfl_sync(kFull, wslot, 0) + __popc(walks & lanemask_lt());
       if (mine) {
+        // what the pair kernel would find out once per pair, here by a lane per pair
+        uint32_t flags = 0;
+        if (t.flat[i] && t.flat[j] && t.nrm[3 * i] == t.nrm[3 * j] && t.nrm[3 * i + 1] == t.nrm[3 * j + 1] &&
+            t.nrm[3 * i + 2] == t.nrm[3 * j + 2])
+          flags |= kOccSame;
+        if (t.mixed) {
+          const double d0 = cj[0] - t.cen[3 * i], d1 = cj[1] - t.cen[3 * i + 1], d2 = cj[2] - t.cen[3 * i + 2];
+          const double dm = fmax(t.diam[i], t.diam[j]) * t.near_factor;
+          if (d0 * d0 + d1 * d1 + d2 * d2 < dm * dm) flags |= kOccNear;
+          if (pair_misses_box<true>(t.cen + 3 * i, cj, fmax(t.rad[i], rj) + t.cull_margin, t.nodes[0]))
+            flags |= kOccOut;
+        }
         OccSlot s;
         s.i = (int32_t)i;
         s.j = (int32_t)j;
-        s.req = s_req;
+        s.req = (int32_t)((uint32_t)s_req | flags);
         s.n = n < 0 ? -1 : n;
         s.off = (int64_t)off;
-        Q.slots[slot] = s;
+        Q.slots[n < 0 ? Q.scap - 1 - (int64_t)wslot : (int64_t)slot] = s;
         n_list += n >= 0 ? 1 : 0;
         n_walk += n < 0 ? 1 : 0;
       }
@@ -756,18 +774,39 @@ __device__ __noinline__ Blocked64 occ_blocked64(const OccArgs& t, int64_t i, int
   return c;
 }
 
+// The warp's FP32 rays by walks of the tree, one ray a lane, the leaf tests
+// dealt out to the lanes (device_trace.cuh): kHit, kMiss or kUnsure.
+__device__ __noinline__ int occ_walk32(const OccArgs& t, bool live, const RayF R, int32_t gi, int32_t gj, RayBankF& ws,
+                                       uint32_t* tests) {
+  PolF3 pol;
+  pol.R = R;
+  pol.tris = t.trisf;
+  TravCount tc;
+  if (live) pol.store(ws, threadIdx.x & 31, gi, gj);
+  const int s = trace_batch(live, GlobalNodes<NodeF>{t.nodesf}, t.n_nodes, ws, pol, tc);
+  tests[0] += tc.nodes;
+  tests[1] += tc.prims;
+  tests[2] += tc.unsure_slab;
+  tests[3] += tc.unsure_prim;
+  return s;
+}
+
 // 3. The queued pairs.  The pair's quadrature points are staged in shared
-// memory, eight values a point.
-template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict__ Lp) {
+// memory, eight values a point.  WALK: the pairs without a list (elements coarse
+// against the obstruction), queued from the other end of the slots; their rays
+// walk the tree.  In a kernel of its own: the walk's code and shared memory cost
+// the list pairs 8 to 16% (closed cube of 43,200 elements).
+template <bool MIXED, bool WALK>
+__global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch* __restrict__ Lp) {
   extern __shared__ __align__(128) unsigned char smem[];
   const OccBatch& B = *Lp;
   const OccQ& Q = B.q;
   const int lane = threadIdx.x & 31;
   using Real = typename std::conditional<MIXED, float, double>::type;
-  Real* Pi = reinterpret_cast<Real*>(smem) + (size_t)(threadIdx.x >> 5) * 16 * B.pmax_max;
+  Real* Pi = reinterpret_cast<Real*>(smem + (WALK ? 8 * sizeof(RayBankF) : 0)) + (size_t)(threadIdx.x >> 5) * 16 * B.pmax_max;
+  uint32_t walk_tests[4] = {0, 0, 0, 0};
   Real* Pj = Pi + 8 * B.pmax_max;
-  const int64_t ns = (int64_t) * (volatile unsigned long long*)(Q.ctr + kCtrSlots);
+  const int64_t ns = (int64_t) * (volatile unsigned long long*)(Q.ctr + (WALK ? kCtrWalk : kCtrSlots));
   // point pairs, rays, FP64 rays, near pairs, grazing point pairs, unusable directions
   uint32_t n_pp = 0, n_rays = 0, n_rays64 = 0, n_near = 0, n_graze = 0, n_bad = 0;
   uint32_t n_nodes = 0, n_prims = 0, n_traced = 0, n_unsure = 0, n_us = 0, n_up = 0;
@@ -776,28 +815,24 @@ __global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict
     // towards the end: lists differ in length by two orders of magnitude
     unsigned long long s0 = 0, len = 1;
     if (lane == 0) {
-      const unsigned long long at = *(volatile unsigned long long*)(Q.ctr + kCtrHead64);
+      const unsigned long long at = *(volatile unsigned long long*)(Q.ctr + (WALK ? kCtrWalkHead : kCtrHead64));
       const unsigned long long left = at < (unsigned long long)ns ? ((unsigned long long)ns - at) / (8ull * gridDim.x * 8) : 0;
       len = left < 1 ? 1 : left > 8 ? 8 : left;
-      s0 = atomicAdd(Q.ctr + kCtrHead64, len);
+      s0 = atomicAdd(Q.ctr + (WALK ? kCtrWalkHead : kCtrHead64), len);
     }
     s0 = __shfl_sync(kFull, s0, 0);
     len = __shfl_sync(kFull, len, 0);
     if ((int64_t)s0 >= ns) break;
     const int64_t s1 = min(ns, (int64_t)(s0 + len));
     for (int64_t s = (int64_t)s0; s < s1; ++s) {
-      const OccSlot ps = Q.slots[s];
-      const OccArgs& t = B.reqs[ps.req];
+      const OccSlot ps = Q.slots[WALK ? Q.scap - 1 - s : s];
+      const OccArgs& t = B.reqs[ps.req & 255];
       const int64_t i = ps.i, j = ps.j, N = t.N;
       const int pm = t.pmax;
       const int64_t oi = t.orig ? (int64_t)t.orig[i] : i, oj = t.orig ? (int64_t)t.orig[j] : j;
       const bool sw = oi > oj;  // the reference casts from the lower caller index
       const int npi = t.np[i];
-      int npj = t.np[j];
-      // elements whose points share one normal, bit for bit, have K = 0
-      if (t.flat[i] && t.flat[j] && t.nrm[3 * i] == t.nrm[3 * j] && t.nrm[3 * i + 1] == t.nrm[3 * j + 1] &&
-          t.nrm[3 * i + 2] == t.nrm[3 * j + 2])
-        npj = 0;
+      const int npj = ps.req & kOccSame ? 0 : t.np[j];  // one normal, bit for bit: K = 0
       const uint32_t* list = Q.pool + ps.off;
       const uint32_t e0 = lane < ps.n ? list[lane] : 0u, e1 = 32 + lane < ps.n ? list[32 + lane] : 0u;
       const NodeF* nodesf = t.nodesf;
@@ -831,11 +866,9 @@ __global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict
           ci[k] = t.cen[3 * i + k];
           dc[k] = t.cen[3 * j + k] - ci[k];
         }
-        const double dm = fmax(t.diam[i], t.diam[j]) * t.near_factor;
-        near = (dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2]) < dm * dm;
+        near = (ps.req & kOccNear) != 0;
         n_near += near && npj > 0 && lane == 0 ? 1 : 0;
-        cullp = pair_misses_box<true>(t.cen + 3 * i, t.cen + 3 * j, fmax(t.rad[i], t.rad[j]) + t.cull_margin,
-                                      t.nodes[0]);
+        cullp = (ps.req & kOccOut) != 0;
       }
       n_pp += lane == 0 ? npi * npj : 0;
       double accd = 0.0;    // the lane's FP64 terms
@@ -939,13 +972,12 @@ __global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict
             if (rok) {
               const int sr = slab_f(nodesf[0], R[u]);
               if (sr != kMiss) {
-                live[u] = sr == kHit && ps.n >= 0;
+                live[u] = sr == kHit;
                 if (!live[u]) st[u] = kUnsure;
                 if (MIXED && !exact) in64[u] = true;  // a ray the root box may hold
                 // mixed: the rays with FP64 terms; FP64: those that pass the root box (the uncertain ones below)
                 n_traced += MIXED ? !exact : sr == kHit;
                 n_us += sr == kUnsure ? 1 : 0;
-                if (sr == kHit && ps.n < 0) st[u] = kUnsure + 1;
               }
             } else {
               st[u] = kUnsure;
@@ -957,7 +989,7 @@ __global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict
         }
         // the pair's list: every lane tests the same box or triangle
         bool open[2] = {live[0], live[1]}, doubt[2] = {false, false};
-        for (int k = 0; k < ps.n; ++k) {
+        for (int k = 0; !WALK && k < ps.n; ++k) {
           if (!__any_sync(kFull, open[0] || open[1])) break;
           const uint32_t e = __shfl_sync(kFull, k < 32 ? e0 : e1, k & 31);
           const NodeF box = nodesf[e >> 8];
@@ -986,6 +1018,16 @@ __global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict
                 doubt[u] = true;
               }
             }
+          }
+        }
+        if constexpr (WALK) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            if (!__any_sync(kFull, live[u])) continue;
+            const int s = occ_walk32(t, live[u], R[u], t.group[i], t.group[j],
+                                     reinterpret_cast<RayBankF*>(smem)[threadIdx.x >> 5], walk_tests);
+            if (live[u] && s == kHit) st[u] = kHit;
+            doubt[u] = s == kUnsure;
           }
         }
         // FP64 for the uncertain rays, one after another
@@ -1032,6 +1074,10 @@ __global__ void __launch_bounds__(256, 2) k_occ_pairs(const OccBatch* __restrict
       __syncwarp();  // before the next pair's points
     }
   }
+  n_nodes += walk_tests[0];
+  n_prims += walk_tests[1];
+  n_us += walk_tests[2];
+  n_up += walk_tests[3];
   if (B.counters) {
     // counters: 0 point pairs, 1 rays, 2 box tests, 3 triangle tests, 4 FP64 rays, 5 near pairs, 6 grazing,
     // 7 unsure rays, 8 / 9 unsure boxes / triangles, 10 unusable directions
@@ -1070,14 +1116,21 @@ cudaError_t launch_occ(bool mixed, int pmax, const OccBatch* b, int list_grid, i
   if (mixed) k_occ_rest<true><<<(unsigned)(2 * sm_count), 256, 0, st>>>(b);
   else k_occ_rest<false><<<(unsigned)(2 * sm_count), 256, stage_bytes(pmax), st>>>(b);
   if ((e = mark(1)) != cudaSuccess) return e;
-  auto pairs = [&](auto fn, size_t smem) -> cudaError_t {
-    const cudaError_t e1 = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e1 != cudaSuccess) return e1;
-    fn<<<(unsigned)(2 * sm_count), 256, smem, st>>>(b);
-    return cudaGetLastError();
+  auto pairs = [&](auto fn, size_t smem, int per_sm) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return;
+    fn<<<(unsigned)(per_sm * sm_count), 256, smem, st>>>(b);
+    e = cudaGetLastError();
   };
-  const size_t points = (size_t)8 * 16 * pmax;  // eight warps, two elements, eight values a point
-  e = mixed ? pairs(k_occ_pairs<true>, points * sizeof(float)) : pairs(k_occ_pairs<false>, points * sizeof(double));
+  // eight warps: eight values a point for two elements, and the walks' ray banks
+  const size_t points = (size_t)8 * 16 * pmax * (mixed ? sizeof(float) : sizeof(double)), bank = 8 * sizeof(RayBankF);
+  if (mixed) {
+    pairs(k_occ_pairs<true, false>, points, 2);
+    pairs(k_occ_pairs<true, true>, bank + points, 3);
+  } else {
+    pairs(k_occ_pairs<false, false>, points, 2);
+    pairs(k_occ_pairs<false, true>, bank + points, 3);
+  }
   if (e != cudaSuccess) return e;
   return mark(2);
 }
