@@ -275,7 +275,10 @@ __device__ __forceinline__ bool mt_d(const TriD& t, const RayD& R) {
   return tt > kTEps && tt < R.tmax;
 }
 
-// 2-D segment blocking test, src/BVH.jl:265-276
+// 2-D segment blocking test, src/BVH.jl:265-276: tol < s < 1 - tol and the same
+// for t, s and t correctly rounded quotients by den.  The comparisons are taken
+// between the numerators and multiples of |den| with a relative margin far above
+// the roundings; only within it are the quotients formed.
 __device__ __forceinline__ bool seg_blocks(const SegD& s, const double* xi, const double* xj) {
   const double tol = 1e-8;
   double dx = xj[0] - xi[0], dy = xj[1] - xi[1];
@@ -283,8 +286,12 @@ __device__ __forceinline__ bool seg_blocks(const SegD& s, const double* xi, cons
   double den = dx * ey - dy * ex;
   if (fabs(den) < tol) return false;
   double fx = s.x0 - xi[0], fy = s.y0 - xi[1];
-  double sp = (fx * ey - fy * ex) / den;
-  double tp = (fx * dy - fy * dx) / den;
+  const double sn = fx * ey - fy * ex, tn = fx * dy - fy * dx;
+  const double a = fabs(den), sa = den < 0.0 ? -sn : sn, ta = den < 0.0 ? -tn : tn;
+  const double lo = fmin(sa, ta), hi = fmax(sa, ta), up = 1.0 - tol;
+  if (lo < (tol * (1.0 - 1e-14)) * a || hi > (up * (1.0 + 1e-14)) * a) return false;
+  if (lo > (tol * (1.0 + 1e-14)) * a && hi < (up * (1.0 - 1e-14)) * a) return true;
+  const double sp = sn / den, tp = tn / den;
   return (tol < sp && sp < 1.0 - tol) && (tol < tp && tp < 1.0 - tol);
 }
 

@@ -192,8 +192,27 @@ __device__ __forceinline__ void stage_row(const double* ib, double* S, int pm) {
   __syncwarp();
 }
 
+// pi K (3-D) or 2 K (2-D) of one point pair, r2 as the shadow rays form it: the
+// fast form, or the reference's cosines where one grazes (their product over the
+// distance needs no correctly rounded quotient).
+template <bool DIM3>
+__device__ __forceinline__ double kernel_scaled(double rx, double ry, double rz, double r2, const double* ni,
+                                                const double* nj) {
+  if (r2 < 1e-30) return 0.0;
+  const double di = fma(ni[0], rx, fma(ni[1], ry, ni[2] * rz));
+  const double dj = -fma(nj[0], rx, fma(nj[1], ry, nj[2] * rz));
+  const double thr = 1e-10 * r2;
+  if (di * di <= thr || dj * dj <= thr) {
+    double ci, cj, r;
+    reference_cosines(rx, ry, rz, r2, ni, nj, ci, cj, r);
+    return ci > 0.0 && cj > 0.0 ? recip_scaled(ci * cj, DIM3 ? r2 : r) : 0.0;
+  }
+  if (di <= 0.0 || dj <= 0.0) return 0.0;
+  return DIM3 ? recip_scaled(di * dj, r2 * r2) : recip32_scaled(di * dj, r2);
+}
+
 // One column (point q of the lane's element, all points p of the source) with
-// k_fast's arithmetic, which takes the reference formula at grazing point pairs.
+// kernel_scaled, which takes the reference formula at grazing point pairs.
 struct ColumnSum {
   double inner;  // scaled as the fast loop's
   uint32_t cast;
@@ -215,21 +234,7 @@ __device__ __noinline__ ColumnSum column_exact(const double* ib, const double* j
     }
     const double rx = xj[0] - xi[0], ry = xj[1] - xi[1], rz = xj[2] - xi[2];
     const double r2 = (rx * rx + ry * ry) + rz * rz;
-    // k_fast's tests; the reference's cosines where one grazes (their product over
-    // r^2 needs no correctly rounded quotient)
-    double k = 0.0;  // pi K (3-D), 2 K (2-D)
-    if (!(r2 < 1e-30)) {
-      const double di = fma(ni[0], rx, fma(ni[1], ry, ni[2] * rz));
-      const double dj = -fma(nj[0], rx, fma(nj[1], ry, nj[2] * rz));
-      const double thr = 1e-10 * r2;
-      if (di * di <= thr || dj * dj <= thr) {
-        double ci, cj, r;
-        reference_cosines(rx, ry, rz, r2, ni, nj, ci, cj, r);
-        if (ci > 0.0 && cj > 0.0) k = recip_scaled(ci * cj, DIM3 ? r2 : r);
-      } else if (di > 0.0 && dj > 0.0) {
-        k = DIM3 ? recip_scaled(di * dj, r2 * r2) : recip32_scaled(di * dj, r2);
-      }
-    }
+    const double k = kernel_scaled<DIM3>(rx, ry, rz, r2, ni, nj);
     s.cast += k > 0.0 ? 1 : 0;
     s.inner = fma(ib[(6 * pm + p) * kTile], -k, s.inner);
   }

@@ -344,6 +344,8 @@ struct OccArgs {
   const TriD* tris;
   const TriF* trisf;
   const float4* sat;
+  const SegD* segs;     // curve meshes
+  double cand_margin;   //   distance beyond which rounding cannot let a segment block a ray
   const int32_t* frontier;
   int n_frontier;
   const int32_t* work;
@@ -379,6 +381,8 @@ struct OccBatch {
   OccQ q;
   unsigned long long* counters;
 };
+// curve meshes with occlusion (kernels_occ2d.cu): every tile, without a queue
+cudaError_t launch_occ2d(int pmax, const OccBatch* b, int sm_count, cudaStream_t st);
 int occ_groups(int64_t n_tiles, int sm_count);
 int occ_list_grid(int sm_count);  // resident blocks of the list kernel
 // marks (or null): events recorded after the list, rest and pair kernels

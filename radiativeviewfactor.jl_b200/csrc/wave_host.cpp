@@ -120,11 +120,11 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   if (o->fault_inject & RVF_FAULT_CLAIM) w.claim_retries = 0;
   w.fast_qb = o->fast_points;
   w.fast_groups = o->fast_row_groups;  // 0: by the tile count (wave_fast)
-  // Surface meshes with occlusion run the occlusion kernels; the queue pipeline
-  // keeps ray logs (every ray's decision in a record), solves without tile
-  // classes, curve meshes and obstructions beyond the lists' 24-bit leaf and
+  // Meshes with occlusion run the occlusion kernels; the queue pipeline keeps
+  // ray logs (every ray's decision in a record), solves without tile classes
+  // and obstructions beyond the lists' 24-bit leaf and
   // 25-bit triangle indices.
-  w.occ_lists = occ && w.dim3 && !o->disable_tile_cull && !ray_log && !(o->fault_inject & RVF_FAULT_CLAIM) &&
+  w.occ_lists = occ && !o->disable_tile_cull && !ray_log && !(o->fault_inject & RVF_FAULT_CLAIM) &&
             m->frontier.ptr && m->n_nodes < (1 << 24) && m->n_obs < (1 << 25);
   PairArgs& a = w.pa;
   a.N = N;
@@ -181,7 +181,7 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
     w.n_tiles = 0;
     w.n_fast_tiles = a.n_tiles;
     w.row_end.assign((size_t)a.nT, 0);
-  } else if (!o->disable_tile_cull && N > 0) {
+  } else if (!o->disable_tile_cull && N > 0 && !(w.occ_lists && !w.dim3)) {  // (curves: every tile is listed)
     int rc = 0;
     const size_t nt = (size_t)a.n_tiles;
     if (T->tcls.bytes < nt && (rc = T->tcls.alloc(s, nt))) return rc;
@@ -276,6 +276,15 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
     x.F = a.F; x.nodes = a.nodes; x.nodesf = ta.nodesf; x.n_nodes = a.n_nodes; x.tris = a.tris; x.trisf = ta.trisf;
     x.sat = ta.sat; x.frontier = ta.frontier; x.n_frontier = ta.n_frontier; x.work = a.work; x.tcls = a.tcls;
     x.tmask = T->tmask.as<uint32_t>();
+    x.segs = a.segs;
+    if (!w.dim3) {
+      // a computed hit of the reference's segment test (src/BVH.jl:265-322: |den| >= 1e-8, parameters strictly inside
+      // (1e-8, 1 - 1e-8)) lies within about 2e-7 S^3 of both segments (S bounds every length)
+      const double S = 2.0 * m->extent;
+      x.cand_margin = 1e-5 * S * S * S + std::ldexp(S, -16);
+      x.frontier = m->frontier.as<int32_t>();
+      x.n_frontier = m->n_frontier;
+    }
   }
   ResolveArgs& ra = w.ra;
   ra.N = N; ra.pmax = a.pmax; ra.dim3 = a.dim3; ra.tab = a.tab; ra.tabf = w.ma.tabf; ra.cen = a.cen;
@@ -381,6 +390,11 @@ cudaError_t enqueue_chunk(Session* s, const WaveShape& sh, bool events) {
   cudaError_t e = cudaMemsetAsync(s->wq_ctr.ptr, 0, sizeof(unsigned long long) * kCtrCount, st);
   if (e != cudaSuccess) return e;
   if (events) cudaEventRecord(s->ev[0], st);
+  if (sh.occ_grid > 0 && !sh.dim3) {
+    if ((e = launch_occ2d(sh.pmax_max, block<OccBatch>(s, kAtOcc), s->sm_count, st)) != cudaSuccess) return e;
+    for (int k = 1; events && k <= 3; ++k) cudaEventRecord(s->ev[k], st);
+    return copy_counters(s);
+  }
   if (sh.occ_grid > 0) {
     if ((e = launch_occ(sh.mixed, sh.pmax_max, block<OccBatch>(s, kAtOcc), sh.occ_grid, s->sm_count, st,
                         events ? &s->ev[1] : nullptr)) != cudaSuccess)
@@ -443,7 +457,11 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   const bool queues = sh.occ && !fused;
   WaveQ q{};
   OccBatch ob{};
-  if (fused) {
+  if (fused && !sh.dim3) {
+    if (!s->wq_ctr.ptr && (rc = s->wq_ctr.alloc(s, sizeof(unsigned long long) * kCtrCount))) return rc;
+    ob.q.ctr = s->wq_ctr.as<unsigned long long>();
+    sh.occ_grid = 1;
+  } else if (fused) {
     if ((rc = ensure_occ(s, base[n], ob.q, sh.occ_grid))) return rc;
   } else if ((rc = ensure_wave(s, sh.mixed && queues, queues, queues && sh.dim3, sh.pmax_max, base[n], q))) {
     return rc;
@@ -482,7 +500,7 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
     ob.pmax_max = sh.pmax_max;
     ob.total_tiles = base[n];
     // a tile is split into tasks only when the queue holds every tile at once
-    const bool all = (base[n] + sh.occ_grid) * kTile * kTile <= ob.q.scap;
+    const bool all = !sh.dim3 || (base[n] + sh.occ_grid) * kTile * kTile <= ob.q.scap;
     ob.groups = all ? occ_groups(base[n], s->sm_count) : 1;
     ob.rest_parts = base[n] * 8 >= (int64_t)64 * s->sm_count ? 8 : 32;
     ob.counters = g.counters;
@@ -536,7 +554,7 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   if (info) {
     *info = ChunkInfo{};
     info->graph = replayed;
-    info->kernels = (fused ? 3 : 1) + (queues ? (sh.mixed ? 3 : 2) + (sh.dim3 ? 1 : 0) : 0);
+    info->kernels = (fused && sh.dim3 ? 4 : 1) + (queues ? (sh.mixed ? 3 : 2) + (sh.dim3 ? 1 : 0) : 0);
     if (!replayed) {
       float t = 0.f;
       cudaEventElapsedTime(&t, s->ev[0], s->ev[1]);
@@ -546,7 +564,7 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
         cudaEventElapsedTime(&tp, s->ev[2], s->ev[3]);
         info->ms_gen = tr;
         info->ms_trace = t + tp;
-        info->ms_lists = t;
+        info->ms_lists = sh.dim3 ? t : 0.0;
       } else {
         info->ms_gen = t;
       }
