@@ -34,6 +34,40 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return r;
 }
 
+// a / b for several a with one b: y = RN(1 / b) (one division), q0 = RN(a y),
+// and twice q <- RN(q + RN(a - q b) y).  The first step leaves q0 (off by at
+// most 2 ulp) faithful, after which the second gives RN(a / b) (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990: a faithful quotient corrected once by the correctly rounded reciprocal
+// is correctly rounded).  The residuals are exact unless a is so small that
+// they underflow: such a (and b out of the middle range) take the division.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = fma(fma(-q0, b, a), y, q0);
+  return fma(fma(-q1, b, a), y, q1);
+}
+// whether a / b may be taken by div_by: a zero or 2^-700 <= |a| < 2^700 (hi words)
+__device__ __forceinline__ bool div_by_ok(double a) {
+  const unsigned h = (unsigned)(__double2hiint(a) & 0x7fffffff);
+  return h - 0x14300000u < 0x57800000u || a == 0.0;
+}
+
+// a / b for N values a, each rounded as the division rounds it
+template <int N>
+__device__ __forceinline__ void div_all(const double (&a)[N], double b, double (&q)[N]) {
+  bool ok = div_by_ok(b);
+#pragma unroll
+  for (int k = 0; k < N; ++k) ok = ok && div_by_ok(a[k]);
+  if (ok) {
+    const double y = 1.0 / b;
+#pragma unroll
+    for (int k = 0; k < N; ++k) q[k] = div_by(a[k], b, y);
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; ++k) q[k] = a[k] / b;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // shape functions, src/GPUKernels.jl:51-176 and src/Geometry.jl:247-334,
 // written in the reference's evaluation order
@@ -104,12 +138,12 @@ __device__ __forceinline__ void eval_surface(const double* __restrict__ coords, 
     ax = ax + dX[k] * cx; ay = ay + dX[k] * cy; az = az + dX[k] * cz;
     bx = bx + dE[k] * cx; by = by + dE[k] * cy; bz = bz + dE[k] * cz;
   }
-  double cx = ay * bz - az * by;
-  double cy = az * bx - ax * bz;
-  double cz = ax * by - ay * bx;
-  double d = sqrt((cx * cx + cy * cy) + cz * cz);
+  const double c[3] = {ay * bz - az * by, az * bx - ax * bz, ax * by - ay * bx};
+  const double d = sqrt((c[0] * c[0] + c[1] * c[1]) + c[2] * c[2]);
   x[0] = px; x[1] = py; x[2] = pz;
-  n[0] = cx / d; n[1] = cy / d; n[2] = cz / d;
+  double u[3];
+  div_all(c, d, u);
+  n[0] = u[0]; n[1] = u[1]; n[2] = u[2];
   *dA = d;
 }
 
@@ -134,51 +168,27 @@ __device__ __forceinline__ void eval_line(const double* __restrict__ coords, con
     tx = tx + dN[k] * xa[0]; ty = ty + dN[k] * xa[1]; tz = tz + dN[k] * xa[2];
   }
   double L = sqrt((tx * tx + ty * ty) + tz * tz);
-  double ux = tx / L, uy = ty / L;
+  const double tt[2] = {tx, ty};
+  double u[2];
+  div_all(tt, L, u);
   x[0] = px; x[1] = py; x[2] = pz;
-  n[0] = -uy; n[1] = ux; n[2] = 0.0;
+  n[0] = -u[1]; n[1] = u[0]; n[2] = 0.0;
   *dL = L;
 }
 
 // ---------------------------------------------------------------------------
 // view-factor kernel
 // ---------------------------------------------------------------------------
-// a / b for several a with one b: y = RN(1 / b) (one division), q0 = RN(a y),
-// and twice q <- RN(q + RN(a - q b) y).  The first step leaves q0 (off by at
-// most 2 ulp) faithful, after which the second gives RN(a / b) (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990: a faithful quotient corrected once by the correctly rounded reciprocal
-// is correctly rounded).  The residuals are exact unless a is so small that
-// they underflow: such a (and b out of the middle range) take the division.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q0 = a * y;
-  const double q1 = fma(fma(-q0, b, a), y, q0);
-  return fma(fma(-q1, b, a), y, q1);
-}
-// whether a / b may be taken by div_by: a zero or 2^-700 <= |a| < 2^700 (hi words)
-__device__ __forceinline__ bool div_by_ok(double a) {
-  const unsigned h = (unsigned)(__double2hiint(a) & 0x7fffffff);
-  return h - 0x14300000u < 0x57800000u || a == 0.0;
-}
-
 // The reference's cosines (src/GPUKernels.jl:204-215 /
 // src/ViewFactorKernel.jl:169-180) and distance, bit for bit.
 __device__ __forceinline__ void reference_cosines(double rx, double ry, double rz, double r2, const double* ni,
                                                   const double* nj, double& ci, double& cj, double& r) {
   r = sqrt(r2);
-  double hx, hy, hz;
-  if (div_by_ok(rx) && div_by_ok(ry) && div_by_ok(rz) && div_by_ok(r)) {
-    const double y = 1.0 / r;
-    hx = div_by(rx, r, y);
-    hy = div_by(ry, r, y);
-    hz = div_by(rz, r, y);
-  } else {
-    hx = rx / r;
-    hy = ry / r;
-    hz = rz / r;
-  }
-  ci = (ni[0] * hx + ni[1] * hy) + ni[2] * hz;
-  cj = (nj[0] * (-hx) + nj[1] * (-hy)) + nj[2] * (-hz);
+  const double rv[3] = {rx, ry, rz};
+  double h[3];
+  div_all(rv, r, h);
+  ci = (ni[0] * h[0] + ni[1] * h[1]) + ni[2] * h[2];
+  cj = (nj[0] * (-h[0]) + nj[1] * (-h[1])) + nj[2] * (-h[2]);
 }
 
 // The reference's kernel, bit for bit.  dim3: cos*cos/(pi r^2); otherwise cos*cos/(2 r).

@@ -459,6 +459,11 @@ struct McArgs {
   const TriD* tris;
   const SegD* segs;
   double cand_margin;  // curves: distance beyond which rounding cannot let a segment block a ray
+  float seg_slack;     //   FP32 rounding of the coordinates in the segment lists' hull tests
+  const NodeF* nodesf;
+  const int32_t* frontier;
+  int n_frontier;
+  int groups;          // tasks per tile (launch_mc)
   const uint8_t* tcls;    // surfaces with occlusion: tile classes and masks (kernels_cull.cu) for the
   const uint32_t* tmask;  //   elements' whole extent, or null (every sample ray walks the tree)
   unsigned long long* tile_counter;

@@ -23,58 +23,10 @@
 
 #include <cstdint>
 
-#include "device_hull.cuh"
 #include "device_pairs.cuh"
+#include "device_segs.cuh"
 
 namespace rvf {
-
-namespace {
-
-constexpr int kSegs = 2048;  // segments of a tile's list
-constexpr int kPairSegs = 24;  // of a pair's (more: its rays walk the tree)
-constexpr int kFront = kTileFront;
-
-struct SegTile {
-  int seg[kSegs];    // segment
-  int leaf[kSegs];   // its leaf node
-  union {
-    struct {
-      int front[2 * kFront];
-      int leaves[kTileLeaves];
-    } walk;
-    uint16_t list[8][kPairSegs][32];  // per warp: the row's pairs' lists (positions in the tile's)
-  };
-};
-
-// True when the hull (of two boxes of FP32 centres and half extents, x and y)
-// is farther than m from the box [lo, hi].
-__device__ __forceinline__ bool hull2_misses(const HullF& H, float lx, float ly, float hx, float hy, float m) {
-  const float ax = fminf(H.c[0][0] - H.h[0][0], H.c[1][0] - H.h[1][0]), bx = fmaxf(H.c[0][0] + H.h[0][0], H.c[1][0] + H.h[1][0]);
-  const float ay = fminf(H.c[0][1] - H.h[0][1], H.c[1][1] - H.h[1][1]), by = fmaxf(H.c[0][1] + H.h[0][1], H.c[1][1] + H.h[1][1]);
-  if (lx - bx > m || ax - hx > m || ly - by > m || ay - hy > m) return true;
-  // the normal of the centroid direction
-  const float wx = -H.d[1], wy = H.d[0];
-  const float bm = 0.5f * ((lx + hx) * wx + (ly + hy) * wy);
-  const float br = 0.5f * ((hx - lx) * fabsf(wx) + (hy - ly) * fabsf(wy));
-  return hull_gap(H, wx, wy, 0.0f, bm - br, bm + br, m);
-}
-
-// True when the segment (s0, s1) is farther than R from the segment a -> a + d
-// (L = |d|), by one of three axes.
-__device__ __forceinline__ bool capsule2_misses(const double* a, const double* d, double L2, double RL, double R,
-                                                const double* s0, const double* s1) {
-  const double u0 = s0[0] - a[0], u1 = s0[1] - a[1], v0 = s1[0] - a[0], v1 = s1[1] - a[1];
-  const double cu = d[0] * u1 - d[1] * u0, cv = d[0] * v1 - d[1] * v0;
-  if (fmin(cu, cv) > RL || fmax(cu, cv) < -RL) return true;
-  const double du = d[0] * u0 + d[1] * u1, dv = d[0] * v0 + d[1] * v1;
-  if (fmax(du, dv) < -RL || fmin(du, dv) > L2 + RL) return true;
-  const double e0 = v0 - u0, e1 = v1 - u1;
-  const double ea = e1 * u0 - e0 * u1, eb = ea - (e1 * d[0] - e0 * d[1]);  // both ends of the centroid segment
-  const double m2 = R * R * (e0 * e0 + e1 * e1);
-  return ((ea > 0.0) == (eb > 0.0)) && fmin(ea * ea, eb * eb) > m2;
-}
-
-}  // namespace
 
 __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ Lp) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -128,72 +80,10 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
     tile_hull(oki, okj, cc, cj, ri, rj, H, rmax, rj_max);
     const int32_t gi0 = __shfl_sync(kFull, gi, 0), gj0 = __shfl_sync(kFull, gj, 0);
     const bool g_same = __all_sync(kFull, (!oki || gi == gi0) && (!okj || gj == gj0));
-    // FP32 coordinates: 2^-20 of the scene's extent
-    const float reach = __double2float_ru(rmax + t.cand_margin) + t.delta;
-    if (warp == 0) {  // the leaves within reach, one tree level per round
-      int* cur = T.walk.front;
-      int* nxt = T.walk.front + kFront;
-      if (lane < t.n_frontier) cur[lane] = t.frontier[lane];
-      __syncwarp();
-      int ncur = t.n_frontier, nleaf = 0;
-      bool over = false;
-      while (ncur > 0 && !over) {
-        int nnext = 0;
-        for (int b = 0; b < ncur; b += 32) {
-          const int q = b + lane;
-          bool pass = false, leaf = false;
-          int k = 0, right = 0;
-          if (q < ncur && cur[q] < t.n_nodes) {
-            k = cur[q];
-            const NodeF nd = t.nodesf[k];
-            pass = !hull2_misses(H, nd.lo[0], nd.lo[1], nd.hi[0], nd.hi[1], reach);
-            leaf = (nd.ab & 15) > 0;
-            if (pass && !leaf) right = t.nodesf[k + 1].miss;
-          }
-          const uint32_t ml = __ballot_sync(kFull, pass && leaf), mi = __ballot_sync(kFull, pass && !leaf);
-          const int pl = nleaf + __popc(ml & lanemask_lt());
-          if (pass && leaf && pl < kTileLeaves) T.walk.leaves[pl] = k;
-          nleaf += __popc(ml);
-          const int pi = nnext + 2 * __popc(mi & lanemask_lt());
-          if (pass && !leaf && pi + 1 < kFront) {
-            nxt[pi] = k + 1;
-            nxt[pi + 1] = right;
-          }
-          nnext += 2 * __popc(mi);
-        }
-        __syncwarp();
-        if (nleaf > kTileLeaves || nnext > kFront) over = true;
-        int* tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        ncur = nnext;
-      }
-      // their segments, four leaves per round
-      int ns = 0;
-      for (int b = 0; b < nleaf && !over; b += 4) {
-        const int li = b + (lane >> 3), u8 = lane & 7;
-        bool keep = false;
-        int leaf = 0, u = 0;
-        if (li < nleaf) {
-          leaf = T.walk.leaves[li];
-          const int32_t ab = t.nodesf[leaf].ab;
-          if (u8 < (ab & 15)) {
-            u = (ab >> 4) + u8;
-            const SegD sg = t.segs[u];
-            const float x0 = (float)sg.x0, y0 = (float)sg.y0, x1 = (float)sg.x1, y1 = (float)sg.y1;
-            keep = !(g_same && (sg.group == gi0 || sg.group == gj0)) &&
-                   !hull2_misses(H, fminf(x0, x1), fminf(y0, y1), fmaxf(x0, x1), fmaxf(y0, y1), reach);
-          }
-        }
-        const uint32_t m = __ballot_sync(kFull, keep);
-        const int at = ns + __popc(m & lanemask_lt());
-        if (keep && at < kSegs) {
-          T.seg[at] = u;
-          T.leaf[at] = leaf;
-        }
-        ns += __popc(m);
-      }
-      if (lane == 0) s_segs = over || ns > kSegs ? -1 : ns;
+    const SegScene sc{t.nodes, t.nodesf, t.n_nodes, t.segs, t.frontier, t.n_frontier, t.cand_margin, t.delta};
+    if (warp == 0) {
+      const int n = tile_segments(sc, H, rmax, g_same, gi0, gj0, T);
+      if (lane == 0) s_segs = n;
     }
     __syncthreads();
     const int nseg = s_segs;
@@ -206,44 +96,8 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
       if (i >= N) break;
       const bool valid = okj && i < j;
       // the lane's pair: its segments, or n = -1 (its rays walk the tree)
-      int n = nseg < 0 && valid ? -1 : 0;
-      if (nseg > 0) {
-        const double A[2] = {t.cen[3 * i], t.cen[3 * i + 1]};
-        const double d[2] = {cj[0] - A[0], cj[1] - A[1]};
-        const double L2 = d[0] * d[0] + d[1] * d[1], R = fmax(t.rad[i], rj) + t.cand_margin, RL = R * sqrt(L2);
-        const int32_t g_i = t.group[i];
-        // the row's own hull: its centroid and the column block's box
-        HullF Hr;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const float l = __double2float_rd(A[k]), h = __double2float_ru(A[k]);
-          Hr.c[0][k] = 0.5f * (l + h);
-          Hr.h[0][k] = 0.5f * (h - l);
-          Hr.c[1][k] = H.c[1][k];
-          Hr.h[1][k] = H.h[1][k];
-          Hr.d[k] = Hr.c[1][k] - Hr.c[0][k];
-        }
-        Hr.c[0][2] = Hr.h[0][2] = Hr.c[1][2] = Hr.h[1][2] = Hr.d[2] = 0.0f;
-        const float row_reach = __double2float_ru(fmax(t.rad[i], rj_max) + t.cand_margin) + t.delta;
-        for (int b = 0; b < nseg; b += 32) {
-          bool keep = false;
-          if (b + lane < nseg) {
-            const SegD sg = t.segs[T.seg[b + lane]];
-            const float x0 = (float)sg.x0, y0 = (float)sg.y0, x1 = (float)sg.x1, y1 = (float)sg.y1;
-            keep = sg.group != g_i &&
-                   !hull2_misses(Hr, fminf(x0, x1), fminf(y0, y1), fmaxf(x0, x1), fmaxf(y0, y1), row_reach);
-          }
-          for (uint32_t m = __ballot_sync(kFull, keep); m; m &= m - 1u) {  // lanes are pairs again
-            const int at = b + __ffs(m) - 1;
-            const SegD sg = t.segs[T.seg[at]];
-            const double s0[2] = {sg.x0, sg.y0}, s1[2] = {sg.x1, sg.y1};
-            if (valid && n >= 0 && sg.group != gj && !capsule2_misses(A, d, L2, RL, R, s0, s1)) {
-              if (n < kPairSegs) T.list[warp][n][lane] = (uint16_t)at;
-              n = n < kPairSegs ? n + 1 : -1;
-            }
-          }
-        }
-      }
+      const double A[3] = {t.cen[3 * i], t.cen[3 * i + 1], 0.0};
+      const int n = pair_segments(sc, H, T, nseg, warp, A, cj, t.rad[i], rj, rj_max, valid, true, t.group[i], gj);
       const bool some = n != 0;
       const uint32_t rest = __ballot_sync(kFull, some);
       fast_fp64<false, true>(a, a.tab + bi * kComp * pm * kTile, S, bi, bj, li + 8, lane, n_pp, n_rays, rest);
@@ -282,14 +136,7 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
           bool blocked = false;
           ++n_traced;
           if (n >= 0) {
-            for (int k = 0; k < n && !blocked; ++k) {
-              const int at = T.list[warp][k][lane];
-              const NodeD& nd = t.nodes[T.leaf[at]];
-              ++n_nodes;
-              if (nd.lo[0] > hx || nd.hi[0] < lx || nd.lo[1] > hy || nd.hi[1] < ly) continue;
-              ++n_prims;
-              blocked = seg_blocks(t.segs[T.seg[at]], from, to);
-            }
+            blocked = list_blocks(sc, T, warp, n, lx, hx, ly, hy, from, to, n_nodes, n_prims);
           } else {
             const int32_t g_i = t.group[i];
             for (int k = 0; k < t.n_nodes && !blocked;) {  // miss links point forward
