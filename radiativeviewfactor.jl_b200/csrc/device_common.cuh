@@ -49,7 +49,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
 // whether a / b may be taken by div_by: a zero or 2^-700 <= |a| < 2^700 (hi words)
 __device__ __forceinline__ bool div_by_ok(double a) {
   const unsigned h = (unsigned)(__double2hiint(a) & 0x7fffffff);
-  return h - 0x14300000u < 0x57800000u || a == 0.0;
+  return h - 0x14300000u < 0x57800000u || (h | (unsigned)__double2loint(a)) == 0u;
 }
 
 // a / b for N values a, each rounded as the division rounds it

@@ -463,7 +463,9 @@ struct McArgs {
   const NodeF* nodesf;
   const int32_t* frontier;
   int n_frontier;
-  int groups;          // tasks per tile (launch_mc)
+  int rows;            // a claim's rows of a tile (launch_mc)
+  const TriF* trisf;      // surfaces with occlusion: FP32 triangles (null: FP64 walks only) and the
+  float delta;            //   rounding of FP32 coordinates
   const uint8_t* tcls;    // surfaces with occlusion: tile classes and masks (kernels_cull.cu) for the
   const uint32_t* tmask;  //   elements' whole extent, or null (every sample ray walks the tree)
   unsigned long long* tile_counter;

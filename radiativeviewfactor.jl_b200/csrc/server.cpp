@@ -466,7 +466,7 @@ void run_mc_chunk(rvf_server* sv, Req* r) {
     c.tile_count = std::min<int64_t>(r->mc_tiles - r->mc_claimed, budget);
     c.area_pass = !r->mc_area_done;
     cudaMemsetAsync(s->err.ptr, 0, sizeof(int), s->stream);
-    cudaMemsetAsync(s->tile_counter.ptr, 0, 8, s->stream);
+    cudaMemsetAsync(s->tile_counter.ptr, 0, 16, s->stream);
     cudaError_t e = launch_mc(c, s->sm_count, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     rc = (e != cudaSuccess) ? cuda_err(e, "Monte Carlo chunk") : read_err(s);

@@ -141,6 +141,10 @@ void fill_mc_args(Session* s, rvf_mesh* m, const rvf_options* o, uint8_t* ray_lo
   }
   c.tcls = (occ && c.dim3 && m->mc_cls_ready) ? m->mc_tcls.as<uint8_t>() : nullptr;
   c.tmask = c.tcls ? m->mc_tmask.as<uint32_t>() : nullptr;
+  if (c.tcls && m->n_obs < (1 << 25)) {  // an FP32 node keeps its first triangle in 28 bits
+    c.trisf = o->geometric_soup ? m->trisf_geo.as<TriF>() : m->trisf_ref.as<TriF>();
+    c.delta = c.seg_slack;
+  }
   c.tile_counter = s->tile_counter.as<unsigned long long>();
   c.counters = s->counters.as<unsigned long long>();
   c.ray_log = ray_log;
@@ -580,7 +584,7 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
   if (m->F.bytes < sizeof(double) * N * N)
     if ((rc = m->F.alloc(s, sizeof(double) * std::max<int64_t>(N * N, 1)))) return rc;
   m->has_result = false;
-  cudaMemsetAsync(s->tile_counter.ptr, 0, 8, s->stream);
+  cudaMemsetAsync(s->tile_counter.ptr, 0, 16, s->stream);
   cudaMemsetAsync(s->counters.ptr, 0, 256, s->stream);
   cudaMemsetAsync(s->err.ptr, 0, sizeof(int), s->stream);
   DevBuf log;
@@ -608,7 +612,7 @@ int rvf_solve(rvf_session* s, rvf_mesh* m, const rvf_options* o, double* F_elem,
       const int t = spans.begin(&S.ms_pairs);
       cudaError_t e = launch_mc(c, s->sm_count, s->stream);
       if (e != cudaSuccess) return cuda_err(e, "Monte Carlo kernel launch");
-      n_kernels += 2;
+      n_kernels += c.dim3 && c.n_nodes > 0 ? 3 : 2;
       spans.end(t);
     }
   } else {
