@@ -22,7 +22,7 @@ struct SegScene {
 };
 
 constexpr int kSegs = 2048;  // segments of a tile's list
-constexpr int kPairSegs = 24;  // of a pair's (more: its rays walk the tree)
+constexpr int kRowItems = 1024;  // (pair, segment) items of a row's pairs (more: its rays walk the tree)
 constexpr int kFront = kTileFront;
 
 struct SegTile {
@@ -33,9 +33,11 @@ struct SegTile {
       int front[2 * kFront];
       int leaves[kTileLeaves];
     } walk;
-    uint16_t list[8][kPairSegs][32];  // per warp: the row's pairs' lists (positions in the tile's)
+    uint16_t item[8][kRowItems];  // per warp: the row's items, position in the tile's list << 5 | lane of the pair
   };
+  double ray[8][4][32];  // per warp: a point pair's rays, from x, y to x, y
 };
+static_assert(kSegs <= 1 << 11, "an item keeps the position in 11 bits");
 
 // True when the hull (of two boxes of FP32 centres and half extents, x and y)
 // is farther than m from the box [lo, hi].
@@ -139,15 +141,18 @@ __device__ __forceinline__ int tile_segments(const SegScene& sc, const HullF& H,
   return over || ns > kSegs ? -1 : ns;
 }
 
-// The lane's pair (row element centre A and radius ri, column element cj, rj):
-// its segments into T.list[warp][..][lane]; their number, or -1 (its rays walk
-// the tree: too many, or no tile list).  skip: rays skip the groups gi, gj.
-// Warp-uniform call.
-__device__ __forceinline__ int pair_segments(const SegScene& sc, const HullF& H, SegTile& T, int nseg, int warp,
-                                             const double* A, const double* cj, double ri, double rj, double rj_max,
-                                             bool valid, bool skip, int32_t gi, int32_t gj) {
+// The segments the row's pairs can be blocked by (lane: row element centre A and
+// radius ri, column element cj, rj) as items in T.item[warp]; their number, or -1
+// (the row's rays walk the tree: too many, or no tile list).  `some`: the pairs
+// with an item (all valid ones when they walk).  skip: rays skip the groups gi, gj.
+// Warp-uniform call and number.
+__device__ __forceinline__ int row_segments(const SegScene& sc, const HullF& H, SegTile& T, int nseg, int warp,
+                                            const double* A, const double* cj, double ri, double rj, double rj_max,
+                                            bool valid, bool skip, int32_t gi, int32_t gj, uint32_t& some) {
   const int lane = threadIdx.x & 31;
-  int n = nseg < 0 && valid ? -1 : 0;
+  some = 0;
+  int n = 0;
+  __syncwarp();  // the last row's items are read
   if (nseg > 0) {
     const double d[2] = {cj[0] - A[0], cj[1] - A[1]};
     const double L2 = d[0] * d[0] + d[1] * d[1], R = fmax(ri, rj) + sc.margin, RL = R * sqrt(L2);
@@ -176,32 +181,56 @@ __device__ __forceinline__ int pair_segments(const SegScene& sc, const HullF& H,
         const int at = b + __ffs(m) - 1;
         const SegD sg = sc.segs[T.seg[at]];
         const double s0[2] = {sg.x0, sg.y0}, s1[2] = {sg.x1, sg.y1};
-        if (valid && n >= 0 && !(skip && sg.group == gj) && !capsule2_misses(A, d, L2, RL, R, s0, s1)) {
-          if (n < kPairSegs) T.list[warp][n][lane] = (uint16_t)at;
-          n = n < kPairSegs ? n + 1 : -1;
-        }
+        const bool in = valid && !(skip && sg.group == gj) && !capsule2_misses(A, d, L2, RL, R, s0, s1);
+        const uint32_t mi = __ballot_sync(kFull, in);
+        const int pos = n + __popc(mi & lanemask_lt());
+        if (in && pos < kRowItems) T.item[warp][pos] = (uint16_t)((at << 5) | lane);
+        n += __popc(mi);
+        some |= mi;
       }
     }
   }
   __syncwarp();
+  if (nseg < 0 || n > kRowItems) {
+    some = __ballot_sync(kFull, valid);
+    return -1;
+  }
   return n;
 }
 
-// Whether a listed segment blocks the ray from -> to with the bounding box
-// [lx, hx] x [ly, hy], each behind the reference's overlap test of its leaf.
-__device__ __forceinline__ bool list_blocks(const SegScene& sc, const SegTile& T, int warp, int n, double lx, double hx,
-                                            double ly, double hy, const double* from, const double* to,
-                                            uint32_t& n_nodes, uint32_t& n_prims) {
+// The lanes (of `cast`) whose ray from -> to is blocked by one of the row's n
+// items, dealt out to the lanes: a lane tests another lane's ray, and the rays'
+// tests of one segment share its load.  The reference tests a segment when the
+// ray's bounding box overlaps its leaf's: looked at for the few hits.
+// Warp-uniform call and result.
+__device__ __forceinline__ uint32_t items_block(const SegScene& sc, SegTile& T, int warp, int n, uint32_t cast,
+                                                const double* from, const double* to, uint32_t& n_nodes,
+                                                uint32_t& n_prims) {
   const int lane = threadIdx.x & 31;
-  for (int k = 0; k < n; ++k) {
-    const int at = T.list[warp][k][lane];
-    const NodeD& nd = sc.nodes[T.leaf[at]];
-    ++n_nodes;
-    if (nd.lo[0] > hx || nd.hi[0] < lx || nd.lo[1] > hy || nd.hi[1] < ly) continue;
-    ++n_prims;
-    if (seg_blocks(sc.segs[T.seg[at]], from, to)) return true;
+  double(*ray)[32] = T.ray[warp];
+  __syncwarp();
+  ray[0][lane] = from[0];
+  ray[1][lane] = from[1];
+  ray[2][lane] = to[0];
+  ray[3][lane] = to[1];
+  __syncwarp();
+  uint32_t blocked = 0;
+  for (int b = 0; b < n; b += 32) {
+    const int item = b + lane < n ? T.item[warp][b + lane] : 0, o = item & 31, at = item >> 5;
+    bool hit = false;
+    if (b + lane < n && (((cast & ~blocked) >> o) & 1u)) {
+      const double f[2] = {ray[0][o], ray[1][o]}, t[2] = {ray[2][o], ray[3][o]};
+      ++n_prims;
+      if (seg_blocks(sc.segs[T.seg[at]], f, t)) {
+        const NodeD& nd = sc.nodes[T.leaf[at]];
+        ++n_nodes;
+        hit = !(nd.lo[0] > fmax(f[0], t[0]) || nd.hi[0] < fmin(f[0], t[0]) || nd.lo[1] > fmax(f[1], t[1]) ||
+                nd.hi[1] < fmin(f[1], t[1]));
+      }
+    }
+    if (__any_sync(kFull, hit)) blocked |= __reduce_or_sync(kFull, hit ? 1u << o : 0u);
   }
-  return false;
+  return blocked;
 }
 
 }  // namespace rvf

@@ -16,6 +16,25 @@
 // xi = 2*((si+u1)/s) - 1, element j at xi = 2*((sj+u3)/s) - 1 (u2, u4 drawn and
 // unused), remainder samples at 2*u1-1 and 2*u3-1, reference measure 2,
 // kernel cos*cos/(2r), occlusion by the 2-D segment test.
+//
+// Surfaces run in two kernels: k_mc_rows, a lane per pair, for the pairs whose
+// rays the tile classification (kernels_cull.cu) proves visible, and k_mc_queue, a
+// lane per sample, for the others.  Curves run in k_mc_curves with per-row segment
+// lists.  Element nodes are staged in shared memory; quotients by a common divisor
+// take one division and a corrected product each (div_by).
+//
+// Measured on a B200, 64 samples a pair.  Closed cube of 2,166 Quad4 with a box:
+// rows 4.4 ms, blockable pairs (7% of all) 5.2 ms, classification 2.9 ms; one kernel
+// with a tree walk in every masked row took 46 ms (2.6 of a row's 32 pairs masked,
+// eight warps at a barrier per tile).  Rows are bound by FP64 issue (66% of the
+// pipe), blockable pairs by the walks' issue and latency.  Cavity of 4,000 Line3 with
+// four circles: 15.5 ms; 33 ms with a tree walk per ray, 24 ms with a lane per
+// pair testing its own list (lists differ in length between the lanes).
+// Measured and not kept: the blockable pairs a lane each (52 ms: a walk's 32 rays
+// share few nodes); per-pair triangle lists in place of the walks (9.4 to 11.0 ms
+// for both kernels by the longest list allowed, against 9.8: a whole element's
+// capsule reaches as many leaves as a walk visits nodes); two blocks a
+// multiprocessor (17.2 ms for the curves).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -143,12 +162,12 @@ struct McStream {
 // R = max(r_i, r_j) of the segment between the elements' centres (each
 // element's points lie within r of its centre).  So a block lists the segments
 // within reach of its tile, a lane per pair those within reach of its capsule
-// (device_segs.cuh), and each sample tests only these, each behind the overlap
-// test of its own leaf (the walk's test at that leaf: the leaf box lies inside
-// every ancestor's, so the test passing there means the reference's walk
-// reaches it), with the reference's own segment test.  Decisions are identical
-// to the full walk's.  Pairs with more than kPairSegs segments, and tiles whose
-// list overflows, walk the tree for every sample.
+// (device_segs.cuh), and each sample tests only these with the reference's own
+// segment test, a hit counting when the overlap test of its leaf passes too (the
+// leaf box lies inside every ancestor's, so the test passing there means the
+// reference's walk reaches it).  Decisions are identical to the full walk's.  Rows
+// with more than kRowItems tests, and tiles whose list overflows, walk the tree for
+// every sample.
 // ---------------------------------------------------------------------------
 
 // Centre and radius of a Line3 / Line2 element: the quadratic curve lies in
@@ -467,7 +486,7 @@ struct McRow {
   double xi[24];
 };
 template <bool OCC>
-__global__ void __launch_bounds__(256, 2) k_mc_rows(McArgs a) {
+__global__ void __launch_bounds__(256, 3) k_mc_rows(McArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   McRow& W = reinterpret_cast<McRow*>(smem)[warp];
@@ -550,7 +569,7 @@ struct McQueue {
   int64_t i[kMcPairs], j[kMcPairs];
   int first[kMcBundle * kTile];      // pairs before each row's
 };
-__global__ void __launch_bounds__(128, 3) k_mc_queue(const __grid_constant__ McArgs a) {
+__global__ void __launch_bounds__(128, 4) k_mc_queue(const __grid_constant__ McArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   McQueue& W = reinterpret_cast<McQueue*>(smem)[warp];
@@ -703,10 +722,11 @@ __global__ void __launch_bounds__(128, 3) k_mc_queue(const __grid_constant__ McA
 // Curves: a block claims a tile or a part of its rows, a warp takes rows, a lane a
 // pair; the elements' nodes in shared memory.
 template <bool OCC, bool FLAT>
-__device__ __forceinline__ void mc_curve_row(const McArgs& a, const SegScene& sc, const SegTile& T, int warp, int ncand,
+__device__ __forceinline__ void mc_curve_row(const McArgs& a, const SegScene& sc, SegTile& T, int warp, int ncand,
                                              const McPair& P, bool valid, int f_i, int f_j, int32_t gi, int32_t gj,
                                              int s, const double* Xi, const double* Xj, uint64_t& n_rays,
                                              TravCount& tc) {
+  const int lane = threadIdx.x & 31;
   McStream q(P.seed(a), s);
   McPoint pi, pj;
   mc_const_tangent(f_i, Xi, 1, pi);
@@ -725,16 +745,17 @@ __device__ __forceinline__ void mc_curve_row(const McArgs& a, const SegScene& sc
       const bool cast = K > 0.0;
       n_rays += cast ? 1 : 0;
       bool blocked = false;
-      if (__any_sync(kFull, cast && ncand != 0)) {
+      const uint32_t casts = ncand != 0 ? __ballot_sync(kFull, cast) : 0u;
+      if (casts) {
         const double from[2] = {P.sw ? pj.x[0] : pi.x[0], P.sw ? pj.x[1] : pi.x[1]};
         const double to[2] = {P.sw ? pi.x[0] : pj.x[0], P.sw ? pi.x[1] : pj.x[1]};
-        const double lx = fmin(from[0], to[0]), hx = fmax(from[0], to[0]);
-        const double ly = fmin(from[1], to[1]), hy = fmax(from[1], to[1]);
-        if (cast && ncand > 0) blocked = list_blocks(sc, T, warp, ncand, lx, hx, ly, hy, from, to, tc.nodes, tc.prims);
-        const bool walk = cast && ncand < 0;
-        if (__any_sync(kFull, walk)) {
-          const bool bw = packet_any_hit(
-              walk, a.nodes, a.n_nodes,
+        if (ncand > 0) {
+          blocked = (items_block(sc, T, warp, ncand, casts, from, to, tc.nodes, tc.prims) >> lane) & 1u;
+        } else {
+          const double lx = fmin(from[0], to[0]), hx = fmax(from[0], to[0]);
+          const double ly = fmin(from[1], to[1]), hy = fmax(from[1], to[1]);
+          blocked = packet_any_hit(
+              cast, a.nodes, a.n_nodes,
               [&](const NodeD& nd) { return !(nd.lo[0] > hx || nd.hi[0] < lx || nd.lo[1] > hy || nd.hi[1] < ly); },
               [&](int kk, bool test) {
                 const SegD sg = a.segs[kk];
@@ -743,7 +764,6 @@ __device__ __forceinline__ void mc_curve_row(const McArgs& a, const SegScene& sc
                 return seg_blocks(sg, from, to);
               },
               tc);
-          if (walk) blocked = bw;
         }
       }
       if (P.log) P.log[k] = cast ? (blocked ? 2 : 1) : 0;
@@ -754,7 +774,7 @@ __device__ __forceinline__ void mc_curve_row(const McArgs& a, const SegScene& sc
   if (valid) P.finish(a, Ks, f_i, f_j);
 }
 template <bool OCC>
-__global__ void __launch_bounds__(256, 2) k_mc_curves(McArgs a) {
+__global__ void __launch_bounds__(256, 3) k_mc_curves(McArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   SegTile& T = *reinterpret_cast<SegTile*>(smem);  // with occlusion
   __shared__ int64_t s_tile;
@@ -839,7 +859,8 @@ __global__ void __launch_bounds__(256, 2) k_mc_curves(McArgs a) {
       if constexpr (OCC) {
         double A[3] = {0.0, 0.0, 0.0}, ri;
         line_bounds(a.coords, a.enodes + 8 * i, f_i, A, ri);
-        ncand = pair_segments(sc, H, T, nseg, warp, A, cj, ri, rj, rj_max, valid, true, gi, gj);
+        uint32_t some;
+        ncand = row_segments(sc, H, T, nseg, warp, A, cj, ri, rj, rj_max, valid, true, gi, gj, some);
       }
       bool flat = true;
 #pragma unroll

@@ -7,18 +7,19 @@
 // hull; row by row, a lane per pair lists those within reach of its own capsule
 // (the segment between the elements' centroids grown by their
 // point radius and by cand_margin, which bounds how far from a ray a computed
-// hit of the segment test can lie).  Pairs with an empty list have visible rays
-// only and run the quadrature-only loop; the others test each ray against their
-// listed segments, each behind the overlap test of its own leaf (the leaf box
-// lies in every ancestor's, so the reference's walk reaches it exactly when it
-// passes), with the reference's segment test: the decisions are the walk's.  A
-// tile with more than kSegs segments within reach, or a pair with more than
-// kPairSegs, walks the tree for every ray.
+// hit of the segment test can lie).  Pairs without one have visible rays only and
+// run the quadrature-only loop; the tests of the others' rays are dealt out to the
+// lanes, with the reference's segment test; a hit counts when the ray's box
+// overlaps the segment's leaf (the leaf box lies in every ancestor's, so the
+// reference's walk reaches it exactly when it does): the decisions are the walk's.
+// A tile with more than kSegs segments within reach, or a row with more than
+// kRowItems tests, walks the tree for every ray.
 //
 // Measured on a B200, 2-D cavity of 4,000 Line3 with four circles of 200 as
-// obstruction, nquad 4: 4.8 ms a solve; walking the tree for every ray took
+// obstruction, nquad 4: 4.2 ms a solve; walking the tree for every ray took
 // 47 ms (39 segment and 16 box tests a ray, from shared memory at 79% of its
-// bandwidth).  Bound by FP64 issue.
+// bandwidth), a lane testing its own pair's list 4.8 ms (lists differ in length
+// between the lanes).  Bound by FP64 issue.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -95,11 +96,11 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
       const int64_t i = bi * kTile + li;
       if (i >= N) break;
       const bool valid = okj && i < j;
-      // the lane's pair: its segments, or n = -1 (its rays walk the tree)
+      // the row's (pair, segment) items, or n = -1 (its rays walk the tree)
       const double A[3] = {t.cen[3 * i], t.cen[3 * i + 1], 0.0};
-      const int n = pair_segments(sc, H, T, nseg, warp, A, cj, t.rad[i], rj, rj_max, valid, true, t.group[i], gj);
-      const bool some = n != 0;
-      const uint32_t rest = __ballot_sync(kFull, some);
+      uint32_t rest;
+      const int n = row_segments(sc, H, T, nseg, warp, A, cj, t.rad[i], rj, rj_max, valid, true, t.group[i], gj, rest);
+      const bool some = (rest >> lane) & 1u;
       fast_fp64<false, true>(a, a.tab + bi * kComp * pm * kTile, S, bi, bj, li + 8, lane, n_pp, n_rays, rest);
       if (rest == 0) continue;  // warp-uniform
       // the pairs with segments in reach (S holds the row's points)
@@ -112,32 +113,38 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
         npj = 0;
       n_pp += (uint32_t)(npi * npj);
       const double* jb = t.tab + bj * kComp * pm * kTile + lane;
+      const int qmax = __reduce_max_sync(kFull, npj);
       double acc = 0.0;  // twice the pair's sum
-      for (int q = 0; q < npj; ++q) {
-        double xj[3], nj[3];
+      for (int q = 0; q < qmax; ++q) {
+        const bool lq = q < npj;
+        double xj[3] = {0.0, 0.0, 0.0}, nj[3] = {0.0, 0.0, 0.0};
+        if (lq) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          xj[c] = jb[(c * pm + q) * kTile];
-          nj[c] = jb[((3 + c) * pm + q) * kTile];
+          for (int c = 0; c < 3; ++c) {
+            xj[c] = jb[(c * pm + q) * kTile];
+            nj[c] = jb[((3 + c) * pm + q) * kTile];
+          }
         }
         double inner = 0.0;
         for (int p = 0; p < npi; ++p) {
           const double xi[3] = {S[8 * p], S[8 * p + 1], S[8 * p + 2]}, ni[3] = {S[8 * p + 4], S[8 * p + 5], S[8 * p + 6]};
           const double rx = xj[0] - xi[0], ry = xj[1] - xi[1], rz = xj[2] - xi[2];
           const double r2 = (rx * rx + ry * ry) + rz * rz;
-          const double k = kernel_scaled<false>(rx, ry, rz, r2, ni, nj);
-          if (!(k > 0.0)) continue;
-          ++n_rays;
-          // the segment as the reference passes it, and its bounding box
-          const double ax = sw ? xj[0] : xi[0], ay = sw ? xj[1] : xi[1], bx = sw ? xi[0] : xj[0],
-                       by = sw ? xi[1] : xj[1];
-          const double lx = fmin(ax, bx), hx = fmax(ax, bx), ly = fmin(ay, by), hy = fmax(ay, by);
-          const double from[2] = {ax, ay}, to[2] = {bx, by};
+          const double k = lq ? kernel_scaled<false>(rx, ry, rz, r2, ni, nj) : 0.0;
+          const bool cast = k > 0.0;
+          const uint32_t casts = __ballot_sync(kFull, cast);
+          if (casts == 0) continue;  // warp-uniform
+          n_rays += cast ? 1 : 0;
+          n_traced += cast ? 1 : 0;
+          // the segment as the reference passes it
+          const double from[2] = {sw ? xj[0] : xi[0], sw ? xj[1] : xi[1]};
+          const double to[2] = {sw ? xi[0] : xj[0], sw ? xi[1] : xj[1]};
           bool blocked = false;
-          ++n_traced;
-          if (n >= 0) {
-            blocked = list_blocks(sc, T, warp, n, lx, hx, ly, hy, from, to, n_nodes, n_prims);
-          } else {
+          if (n > 0) {
+            blocked = (items_block(sc, T, warp, n, casts, from, to, n_nodes, n_prims) >> lane) & 1u;
+          } else if (cast) {
+            const double lx = fmin(from[0], to[0]), hx = fmax(from[0], to[0]);
+            const double ly = fmin(from[1], to[1]), hy = fmax(from[1], to[1]);
             const int32_t g_i = t.group[i];
             for (int k = 0; k < t.n_nodes && !blocked;) {  // miss links point forward
               const NodeD nd = t.nodes[k];
@@ -155,9 +162,9 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
               k = nd.b > 0 ? nd.miss : k + 1;
             }
           }
-          if (!blocked) inner = fma(S[8 * p + 3], k, inner);
+          if (cast && !blocked) inner = fma(S[8 * p + 3], k, inner);
         }
-        acc = fma(jb[(6 * pm + q) * kTile], inner, acc);
+        if (lq) acc = fma(jb[(6 * pm + q) * kTile], inner, acc);
       }
       if (some) {
         const double raw = 0.5 * acc;
