@@ -79,26 +79,44 @@ __device__ __forceinline__ int slab_f(const NodeF& nd, const RayF& R) {
   return slack > m ? kHit : slack < -m ? kMiss : kUnsure;
 }
 
+// Allowances of mt_f: e0 relative (|o - v0| |e| or |e1| |e2|), d absolute, in
+// units of the ray's delta = 2^-20 extent.
+struct MtTol {
+  float e0, d;
+};
+constexpr MtTol kMtLoose{kE0, 2.0f};
+// For rays whose direction is off by at most 7 2^-24 in each component: r formed
+// in FP64 and rounded, or as (c_j - c_i) + (o_q - o_p) in FP32 with the centroids
+// at least two diameters apart (|r| >= 0.4 |c_j - c_i|, |o| <= 0.6 diameters:
+// 2^-24 (2.5 + 3 + 1), and the scaling's rounding).  With u = 2^-24, ns = |s|_1:
+// h = d x e2 is within 13.4 u n2 a component, so U = s.h within
+// (13.4 + 3 + 1) u ns n2 = 2^-19.9 ns n2, V within (1.73 4.5 + 12 + 5) u ns n1 =
+// 2^-19.4 ns n1, T within 14.5 u ns n1 n2 and a within 30 u n1 n2 = 2^-19.1 n1 n2:
+// 2^-18 is twice the largest.  Positions (origin 2^-23, vertex 2^-24 of the
+// coordinates) move U by at most 4.5 2^-23 n2 = 2^-20.8 n2 and V by 2^-20.6 n1 per unit
+// extent, against 2^-19.7 and 2^-18.7 here.
+constexpr MtTol kMtTight{3.814697265625e-06f, 1.25f};
+
 // Moller-Trumbore with certified outcome; the triangle stores |e1|, |e2|
 // (rounded up) in n1, n2.  The reference's u, v, t are quotients U / a, V / a,
 // T / a; with |a| certainly above its cut, each comparison is taken between
 // the numerators and multiples of |a| (no division), the numerators within
-//   |dU| <= (kE0 ns + d2) n2,  |dV| <= (kE0 ns + 2 d2) n1,  |dT| <= (kE0 ns + 2 d2) n1 n2
-// and |da| <= kE0 n1 n2 of the reference's (ns bounds |o - v0|, d2 = 2 delta;
+//   |dU| <= (e0 ns + d2) n2,  |dV| <= (e0 ns + 2 d2) n1,  |dT| <= (e0 ns + 2 d2) n1 n2
+// and |da| <= e0 n1 n2 of the reference's (ns bounds |o - v0|, d2 = d delta;
 // the relative terms also cover its own FP64 rounding).
-__device__ __forceinline__ int mt_f(const TriF& t, const RayF& R) {
+__device__ __forceinline__ int mt_f(const TriF& t, const RayF& R, MtTol tol = kMtLoose) {
   const float n1 = __int_as_float(t.pad0), n2 = __int_as_float(t.pad1);
   const float hx = fmaf(R.d[1], t.e2[2], -R.d[2] * t.e2[1]);
   const float hy = fmaf(R.d[2], t.e2[0], -R.d[0] * t.e2[2]);
   const float hz = fmaf(R.d[0], t.e2[1], -R.d[1] * t.e2[0]);
   const float a = fmaf(t.e1[0], hx, fmaf(t.e1[1], hy, t.e1[2] * hz));
-  const float na = n1 * n2, Ea = kE0 * na;
+  const float na = n1 * n2, Ea = tol.e0 * na;
   const float aa = fabsf(a), hi = aa + Ea, lo = aa - Ea;
   if (hi < 1e-10f) return kMiss;
   if (lo < 1e-10f) return kUnsure;
   const float sx = R.o[0] - t.v0[0], sy = R.o[1] - t.v0[1], sz = R.o[2] - t.v0[2];
-  const float d2 = 2.0f * R.delta;
-  const float e = fmaf(kE0, fabsf(sx) + fabsf(sy) + fabsf(sz) + d2, d2), e2 = e + d2;
+  const float d2 = tol.d * R.delta;
+  const float e = fmaf(tol.e0, fabsf(sx) + fabsf(sy) + fabsf(sz) + d2, d2), e2 = e + d2;
   const float u = copysignf(1.0f, a) * fmaf(sx, hx, fmaf(sy, hy, sz * hz));
   const float cu = e * n2;
   if (u < -cu || u > hi + cu) return kMiss;
@@ -111,9 +129,9 @@ __device__ __forceinline__ int mt_f(const TriF& t, const RayF& R) {
   const float w = copysignf(1.0f, a) * fmaf(t.e2[0], qx, fmaf(t.e2[1], qy, t.e2[2] * qz));
   const float cw = e2 * na;
   const float eps = (float)kTEps, tm = 2.0f * kRho * R.tmax;
-  if (w + cw < (1.0f - kE0) * eps * lo || w - cw > (R.tmax + tm) * hi) return kMiss;
+  if (w + cw < (1.0f - tol.e0) * eps * lo || w - cw > (R.tmax + tm) * hi) return kMiss;
   const bool inside = u > cu && u < lo - cu && v > cv && u + v < lo - cuv;
-  return inside && w - cw > (1.0f + kE0) * eps * hi && w + cw < (R.tmax - tm) * lo ? kHit : kUnsure;
+  return inside && w - cw > (1.0f + tol.e0) * eps * hi && w + cw < (R.tmax - tm) * lo ? kHit : kUnsure;
 }
 
 // Warp-coherent FP32 any-hit traversal (same walk as packet_any_hit) with

@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(128, 4) k_mc_queue(const __grid_constant__ McA
                     const TriF tr = a.trisf[kk];
                     if (!test || tr.group == gx || tr.group == gy) return kMiss;
                     ++tc.prims;
-                    return mt_f(tr, R);
+                    return mt_f(tr, R, kMtTight);
                   },
                   unsure, tc);
               again = cast && (unsure || !usable);

@@ -838,6 +838,7 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
       const NodeF* nodesf = t.nodesf;
       const TriF* trisf = t.trisf;
       const float delta = t.delta;
+      const MtTol tol = !MIXED || t.near_factor >= 2.0 ? kMtTight : kMtLoose;
       const double* it = t.tab + tab_at(i, 0, 0, pm);
       const double* jt = t.tab + tab_at(j, 0, 0, pm);
       const float per = 1.0f / (float)pm;  // v + 1/2 is at least 1/128 from a multiple of pm, v < 448
@@ -1008,7 +1009,7 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
             for (int u = 0; u < 2; ++u) {
               if (sb[u] == kMiss) continue;
               ++n_prims;
-              const int h = mt_f(tr, R[u]);
+              const int h = mt_f(tr, R[u], tol);
               n_up += h == kUnsure ? 1 : 0;
               if (h == kHit && sb[u] == kHit) {
                 st[u] = kHit;
