@@ -444,6 +444,179 @@ __device__ __forceinline__ void gen_fast_mixed_body(const MixedArgs& a, const fl
   }
 }
 
+// Two FP32 values in a register pair: one instruction does both operations, each
+// rounded as the scalar one.
+using F32x2 = unsigned long long;
+__device__ __forceinline__ F32x2 f2_pack(float x, float y) {
+  F32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(F32x2 a, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+}
+__device__ __forceinline__ F32x2 f2_add(F32x2 a, F32x2 b) {
+  F32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F32x2 f2_mul(F32x2 a, F32x2 b) {
+  F32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F32x2 f2_fma(F32x2 a, F32x2 b, F32x2 c) {
+  F32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// The same in the kernel that only does this:
+// two of the column's points per instruction (packed FP32), the row's points in
+// shared memory S with every value twice, so that an operand is a load, and the
+// column's points kept in registers over the rows when one block holds them.  Every
+// operation rounds as in gen_fast_mixed_body.  Bound by the FP32 pipes' non-packed
+// operations (comparisons, selections, reciprocals).  Closed cube of 43,200 Tri3, 7
+// points, the tiles without ray work: 56.1 ms with gen_fast_mixed_body, 55 with
+// packed operations alone (long waits for the row's points from global memory), 44 ms
+// so; single rows (k_occ_rest) gain nothing (+5 of 16 ms).
+template <bool OCC, int QB>
+__device__ __forceinline__ void fast_mixed_rows(const MixedArgs& a, const float* iblk, double* S, int64_t bi, int64_t bj,
+                                                int li0, int lane, uint32_t& n_pp, uint32_t& n_rays) {
+  const int64_t N = a.N;
+  const int pm = a.pmax;
+  const int64_t j = bj * kTile + lane;
+  const bool jok = j < N;
+  const int64_t oj = jok ? (a.orig ? (int64_t)a.orig[j] : j) : 0;
+  const int npj0 = jok ? a.np[j] : 0;
+  const float* jbf = a.tabf + bj * kComp * pm * kTile + lane;
+  const double cj0 = jok ? a.cen[3 * j] : 0.0, cj1 = jok ? a.cen[3 * j + 1] : 0.0, cj2 = jok ? a.cen[3 * j + 2] : 0.0;
+  // The column element's points in pairs, the last one alone when QB is odd;
+  // normals negated (so is dj, exactly).  One block of points holds them all: loaded
+  // once for the tile's rows.
+  constexpr int P = QB / 2;
+  F32x2 oq[P][3], nq[P][3];
+  float wq[QB], oqs[3] = {0.0f, 0.0f, 0.0f}, nqs[3] = {0.0f, 0.0f, 0.0f};
+  auto load = [&](int q0) {
+    auto at = [&](int c, int u) { return q0 + u < npj0 ? jbf[(c * pm + q0 + u) * kTile] : 0.0f; };
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int u = 0; u < P; ++u) {
+        oq[u][c] = f2_pack(at(c, 2 * u), at(c, 2 * u + 1));
+        nq[u][c] = f2_pack(-at(3 + c, 2 * u), -at(3 + c, 2 * u + 1));
+      }
+      if (QB & 1) {
+        oqs[c] = at(c, QB - 1);
+        nqs[c] = -at(3 + c, QB - 1);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < QB; ++u) wq[u] = at(6, u);
+  };
+  if (pm <= QB) load(0);
+  const F32x2 pi2 = f2_pack(3.14159265f, 3.14159265f);
+  // li0 < 8: the warp's rows li0, li0 + 8, ...; li0 >= 8: the single row li0 - 8
+  for (int li = li0 < 8 ? li0 : li0 - 8; li < kTile; li += li0 < 8 ? 8 : kTile) {
+    const int64_t i = bi * kTile + li;
+    if (i >= N) break;  // warp-uniform
+    const bool valid = jok && i < j;
+    const int64_t oi = a.orig ? (int64_t)a.orig[i] : i;
+    const int npi = a.np[i];
+    int npj = valid ? npj0 : 0;
+    if (valid && a.flat[i] && a.flat[j] && a.nrm[3 * i] == a.nrm[3 * j] && a.nrm[3 * i + 1] == a.nrm[3 * j + 1] &&
+        a.nrm[3 * i + 2] == a.nrm[3 * j + 2])
+      npj = 0;
+    const int qmax = __reduce_max_sync(kFull, npj);
+    const float d0 = (float)(cj0 - a.cen[3 * i]), d1 = (float)(cj1 - a.cen[3 * i + 1]),
+                d2 = (float)(cj2 - a.cen[3 * i + 2]);
+    // the row's points, every value twice: -o0 | -o1 | -o2 | n0 | n1 | n2 | w
+    const float* ibf = iblk + li;
+    float4* Sf = reinterpret_cast<float4*>(S);
+    __syncwarp();
+    for (int p = lane; p < npi; p += 32) {
+      float v[7];
+#pragma unroll
+      for (int c = 0; c < 7; ++c) v[c] = ibf[(c * pm + p) * kTile];
+      Sf[4 * p] = make_float4(-v[0], -v[0], -v[1], -v[1]);
+      Sf[4 * p + 1] = make_float4(-v[2], -v[2], v[3], v[3]);
+      Sf[4 * p + 2] = make_float4(v[4], v[4], v[5], v[5]);
+      Sf[4 * p + 3] = make_float4(v[6], v[6], 0.0f, 0.0f);
+    }
+    __syncwarp();
+    float acc32 = 0.0f;
+    uint32_t cast = 0;
+    const F32x2 d02 = f2_pack(d0, d0), d12 = f2_pack(d1, d1), d22 = f2_pack(d2, d2);
+    for (int q0 = 0; q0 < qmax; q0 += QB) {
+      if (pm > QB) load(q0);
+      F32x2 inner2[P];
+      float inners = 0.0f;
+#pragma unroll
+      for (int u = 0; u < P; ++u) inner2[u] = f2_pack(0.0f, 0.0f);
+      for (int p = 0; p < npi; ++p) {
+        const ulonglong2* sp = reinterpret_cast<const ulonglong2*>(S) + 4 * p;
+        const ulonglong2 s0 = sp[0], s1 = sp[1], s2 = sp[2];
+        const F32x2 o0 = s0.x, o1 = s0.y, o2 = s1.x, n0 = s1.y, n1 = s2.x, n2 = s2.y, w2 = sp[3].x;
+        // straight-line over the block: a point q0 + u >= npj has zero
+        // normal, so its dj is 0 and its K zero
+#pragma unroll
+        for (int u = 0; u < P; ++u) {
+          const F32x2 rx = f2_add(d02, f2_add(oq[u][0], o0)), ry = f2_add(d12, f2_add(oq[u][1], o1)),
+                      rz = f2_add(d22, f2_add(oq[u][2], o2));
+          const F32x2 r2 = f2_fma(rx, rx, f2_fma(ry, ry, f2_mul(rz, rz)));
+          const F32x2 di = f2_fma(n0, rx, f2_fma(n1, ry, f2_mul(n2, rz)));
+          const F32x2 dj = f2_fma(nq[u][0], rx, f2_fma(nq[u][1], ry, f2_mul(nq[u][2], rz)));
+          float b0, b1, k0, k1, i0, i1, j0, j1;
+          f2_unpack(f2_mul(pi2, f2_mul(r2, r2)), b0, b1);
+          f2_unpack(f2_mul(f2_mul(di, dj), f2_pack(rcp_approx(b0), rcp_approx(b1))), k0, k1);
+          f2_unpack(di, i0, i1);
+          f2_unpack(dj, j0, j1);
+          k0 = i0 > 0.0f && j0 > 0.0f ? k0 : 0.0f;
+          k1 = i1 > 0.0f && j1 > 0.0f ? k1 : 0.0f;
+          cast += k0 > 0.0f ? 1 : 0;
+          cast += k1 > 0.0f ? 1 : 0;
+          inner2[u] = f2_fma(w2, f2_pack(k0, k1), inner2[u]);
+        }
+        if (QB & 1) {
+          float op0, op1, op2, np0, np1, np2, wp, skip2;
+          f2_unpack(o0, op0, skip2);
+          f2_unpack(o1, op1, skip2);
+          f2_unpack(o2, op2, skip2);
+          f2_unpack(n0, np0, skip2);
+          f2_unpack(n1, np1, skip2);
+          f2_unpack(n2, np2, skip2);
+          f2_unpack(w2, wp, skip2);
+          const float rx = d0 + (oqs[0] + op0), ry = d1 + (oqs[1] + op1), rz = d2 + (oqs[2] + op2);
+          const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+          const float di = fmaf(np0, rx, fmaf(np1, ry, np2 * rz));
+          const float dj = fmaf(nqs[0], rx, fmaf(nqs[1], ry, nqs[2] * rz));
+          const float K32 = (di > 0.0f && dj > 0.0f) ? (di * dj) * rcp_approx(3.14159265f * (r2 * r2)) : 0.0f;
+          cast += K32 > 0.0f ? 1 : 0;
+          inners = fmaf(wp, K32, inners);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < QB; ++u) {
+        float v = inners, x, y;
+        if (u < 2 * P) {
+          f2_unpack(inner2[u / 2], x, y);
+          v = u & 1 ? y : x;
+        }
+        if (q0 + u < npj) acc32 = fmaf(wq[u], v, acc32);
+      }
+    }
+    if (OCC) n_rays += npj > 0 ? cast : 0u;
+    n_pp += (uint32_t)(npi * npj);
+    const double raw = 0.0 + (double)acc32;
+    if (valid) {
+      a.F[oi + oj * N] = raw / a.area[i];
+      a.F[oj + oi * N] = raw / a.area[j];
+    } else if (j == i) {
+      a.F[oi + oi * N] = 0.0 / a.area[i];
+    }
+  }
+}
+
 // Out of line inside the chunked generation kernels, whose own registers are
 // allocated for the ray pipeline.
 template <bool DIM3, bool OCC, int QB>

@@ -1268,6 +1268,8 @@ __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_fp64(const Pa
 template <bool OCC, int QB>
 __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_mixed(const MixedArgs a, unsigned long long* task_ctr,
                                                                         unsigned long long* counters) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  double* S = reinterpret_cast<double*>(smem) + (threadIdx.x >> 5) * 8 * a.pmax;
   const int lane = threadIdx.x & 31;
   uint32_t n_pp = 0, n_rays = 0;
   int64_t t;
@@ -1276,7 +1278,7 @@ __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_mixed(const M
     int64_t bi, bj;
     tile_coords(t, a.nT, bi, bj);
     const float* ib = a.tabf + bi * kComp * a.pmax * kTile;
-    for (int r = r0; r < r1; ++r) gen_fast_mixed_body<OCC, QB>(a, ib, bi, bj, r, lane, n_pp, n_rays);
+    for (int r = r0; r < r1; ++r) fast_mixed_rows<OCC, QB>(a, ib, S, bi, bj, r, lane, n_pp, n_rays);
   }
   const uint64_t s_pp = warp_sum_u64(n_pp), s_rays = warp_sum_u64(n_rays);
   if (lane == 0 && counters) {
@@ -1326,7 +1328,7 @@ cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs&
                         unsigned long long* task_ctr, unsigned long long* counters, int sm_count, cudaStream_t st) {
   auto launch = [&](auto fn, const auto& args) -> cudaError_t {
     int per_sm = 1;
-    const size_t smem = mixed ? 0 : stage_bytes(a.pmax);
+    const size_t smem = stage_bytes(mixed ? m.pmax : a.pmax);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
     fn<<<(unsigned)(sm_count * per_sm), 256, smem, st>>>(args, task_ctr, counters);
     return cudaGetLastError();
