@@ -241,7 +241,8 @@ __device__ __noinline__ ColumnSum column_exact(const double* ib, const double* j
   return s;
 }
 
-template <bool DIM3, bool OCC, int QB>
+// PLANE: pairs of plane elements by flat_fp64 first.
+template <bool DIM3, bool OCC, int QB, bool PLANE = DIM3>
 __device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const double* iblk, double* S, int64_t bi,
                                                    int64_t bj, int li0, int lane, uint32_t& n_pp, uint32_t& n_rays,
                                                    uint32_t skip = 0) {
@@ -278,7 +279,7 @@ __device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const doub
     stage_row(ib, S, pm);
     double acc = 0.0;  // minus pi (3-D) or 2 (2-D) times the pair's sum
     n_pp += (uint32_t)(npi * npj);
-    if constexpr (DIM3) {
+    if constexpr (PLANE) {
       const int npf = npj > 0 && a.flat[i] && a.flat[j] && d2 > 64.0 * s2 ? npj : 0;
       if (__any_sync(kFull, npf > 0)) {
         const FlatSum f = flat_fp64(S, jb, pm, npi, npf, 1.27e-6 * d2);
@@ -357,6 +358,128 @@ __device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const doub
     } else if (j == i) {
       a.F[oi + oi * N] = 0.0 / a.area[i];
     }
+  }
+}
+
+// a / b with y = 1 / b, rounded as the division
+__device__ __forceinline__ double div_or(double a, double b, double y) {
+  return div_by_ok(a) && div_by_ok(b) ? div_by(a, b, y) : a / b;
+}
+
+// The pairs of plane elements (flat_fp64) in the rows li0, li0 + 8, ... of a tile,
+// for rules of at most QB points, in the kernel that only does this: the column's
+// points are loaded once for the rows, which are staged together, and a row of pairs
+// that are all done needs nothing else; the other rows run the general loop for what
+// is left.  Same sums, bit for bit.  Bound by latency and FP64 issue.  Closed cube of
+// 43,200 Tri3, 7 points, the tiles without ray work: 75 ms with flat_fp64 row by row
+// (stalls on the column's points), 60 ms so.
+constexpr int kFlatRows = kTile / 8, kFlatPoints = 7;
+template <bool OCC, int QB>
+__device__ __forceinline__ void flat_rows(const PairArgs& a, const double* iblk, double* S, int64_t bi, int64_t bj,
+                                          int li0, int lane, uint32_t& n_pp, uint32_t& n_rays) {
+  const int64_t N = a.N;
+  const int pm = a.pmax;
+  const int64_t j = bj * kTile + lane, e = j < N ? j : bj * kTile;
+  const bool jok = j < N;
+  const int64_t oj = a.orig ? (int64_t)a.orig[e] : e;
+  const int npj = jok ? a.np[j] : 0;
+  const bool flat_j = a.flat[e];
+  uint32_t left[kFlatRows] = {kFull, kFull, kFull, kFull};  // pairs the general loop takes
+  if (__any_sync(kFull, flat_j)) {
+    const double* jb = a.tab + bj * kComp * pm * kTile + (jok ? lane : 0);
+    const double mj[3] = {a.nrm[3 * e], a.nrm[3 * e + 1], a.nrm[3 * e + 2]};
+    const double cj[3] = {a.cen[3 * e], a.cen[3 * e + 1], a.cen[3 * e + 2]};
+    const double rj = a.rad[e], aj = a.area[e], yj = 1.0 / aj;
+    double x[QB][3], nj[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      nj[c] = jb[(3 + c) * pm * kTile];
+#pragma unroll
+      for (int u = 0; u < QB; ++u) x[u][c] = jb[(c * pm + (u < npj ? u : 0)) * kTile];  // past them: not summed
+    }
+    __syncwarp();
+    for (int v = lane; v < kFlatRows * pm; v += 32) {
+      const int rr = v / pm, q = v - rr * pm, li = li0 + 8 * rr;
+      double* s = S + 8 * v;
+      const double* ib = iblk + li + q * kTile;
+#pragma unroll
+      for (int c = 0; c < kComp; ++c) s[c < 3 ? c : c == 6 ? 3 : c + 1] = ib[c * pm * kTile];
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int rr = 0; rr < kFlatRows; ++rr) {
+      const int li = li0 + 8 * rr;
+      const int64_t i = bi * kTile + li;
+      if (i >= N) continue;  // warp-uniform
+      const double* Sr = S + 8 * rr * pm;
+      const bool valid = jok && i < j;
+      const double dx = cj[0] - a.cen[3 * i], dy = cj[1] - a.cen[3 * i + 1], dz = cj[2] - a.cen[3 * i + 2];
+      const double s = a.rad[i] + rj, d2 = dx * dx + dy * dy + dz * dz;
+      const bool flat_i = a.flat[i];
+      const bool same =
+          flat_i && flat_j && a.nrm[3 * i] == mj[0] && a.nrm[3 * i + 1] == mj[1] && a.nrm[3 * i + 2] == mj[2];
+      bool ok = valid && flat_i && flat_j && npj > 0 && !same && d2 > 64.0 * (s * s);
+      if (__any_sync(kFull, ok)) {
+        const int npi = a.np[i];
+        const double limit = 1.27e-6 * d2;
+        double inner[QB];
+#pragma unroll
+        for (int u = 0; u < QB; ++u) inner[u] = 0.0;
+        int pos_i = 0, pos_j = 0;
+        for (int p = 0; p < npi; ++p) {
+          const double2* sp = reinterpret_cast<const double2*>(Sr + 8 * p);
+          const double2 s0 = sp[0], s1 = sp[1];
+          const double x0 = s0.x, x1 = s0.y, x2 = s1.x;
+          const double dj = fma(nj[0], x0 - x[0][0], fma(nj[1], x1 - x[0][1], nj[2] * (x2 - x[0][2])));
+          const bool facing = __double2hiint(dj) >= 0;
+          const double w = facing ? s1.y * dj : 0.0;
+          ok = ok && dj * dj > limit;
+          pos_j += facing ? 1 : 0;
+#pragma unroll
+          for (int u = 0; u < QB; ++u) {
+            const double rx = x[u][0] - x0, ry = x[u][1] - x1, rz = x[u][2] - x2;
+            const double r2 = fma(rx, rx, fma(ry, ry, rz * rz)), r4 = r2 * r2;
+            double y;
+            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r4));
+            const double er = fma(-r4, y, 1.0);
+            inner[u] = fma(w, fma(y, fma(er, er, er), y), inner[u]);
+          }
+        }
+        double acc = 0.0;
+        const double xi[3] = {Sr[0], Sr[1], Sr[2]}, ni[3] = {Sr[4], Sr[5], Sr[6]};
+#pragma unroll
+        for (int u = 0; u < QB; ++u) {
+          if (u < npj) {
+            const double di = fma(ni[0], x[u][0] - xi[0], fma(ni[1], x[u][1] - xi[1], ni[2] * (x[u][2] - xi[2])));
+            ok = ok && di * di > limit;
+            if (__double2hiint(di) >= 0) {
+              acc = fma(jb[(6 * pm + u) * kTile] * di, inner[u], acc);
+              ++pos_i;
+            }
+          }
+        }
+        if (ok) {
+          n_pp += (uint32_t)(npi * npj);
+          if (OCC) n_rays += (uint32_t)(pos_i * pos_j);
+          const double raw = acc * (1.0 / kPiD), ai = a.area[i];
+          const int64_t oi = a.orig ? (int64_t)a.orig[i] : i;
+          a.F[oi + oj * N] = div_or(raw, ai, 1.0 / ai);
+          a.F[oj + oi * N] = div_or(raw, aj, yj);
+        }
+      }
+      const uint32_t m = __ballot_sync(kFull, jok && i <= j && !ok);
+      left[0] = rr == 0 ? m : left[0];
+      left[1] = rr == 1 ? m : left[1];
+      left[2] = rr == 2 ? m : left[2];
+      left[3] = rr == 3 ? m : left[3];
+    }
+  }
+#pragma unroll 1
+  for (int rr = 0; rr < kFlatRows; ++rr) {
+    const uint32_t m = rr == 0 ? left[0] : rr == 1 ? left[1] : rr == 2 ? left[2] : left[3];
+    const int li = li0 + 8 * rr;
+    if (m && bi * kTile + li < N)
+      gen_fast_fp64_body<true, OCC, (QB < 4 ? 3 : 4), false>(a, iblk, S, bi, bj, 8 + li, lane, n_pp, n_rays, ~m);
   }
 }
 

@@ -1265,6 +1265,29 @@ __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_fp64(const Pa
   }
 }
 
+// Surfaces, rules of at most QB <= 7 points: pairs of plane elements by flat_rows.
+template <bool OCC, int QB>
+__global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_flat(const PairArgs a, unsigned long long* task_ctr,
+                                                                       unsigned long long* counters) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  double* S = reinterpret_cast<double*>(smem) + (threadIdx.x >> 5) * kFlatRows * 8 * a.pmax;
+  const int lane = threadIdx.x & 31;
+  uint32_t n_pp = 0, n_rays = 0;
+  int64_t t;
+  int r0, r1;
+  while (fast_task(task_ctr, a.n_tiles, a.fast_groups, a.tcls, kClsSlow, lane, t, r0, r1)) {
+    int64_t bi, bj;
+    tile_coords(t, a.nT, bi, bj);
+    const double* ib = a.tab + bi * kComp * a.pmax * kTile;
+    for (int r = r0; r < r1; ++r) flat_rows<OCC, QB>(a, ib, S, bi, bj, r, lane, n_pp, n_rays);
+  }
+  const uint64_t s_pp = warp_sum_u64(n_pp), s_rays = warp_sum_u64(n_rays);
+  if (lane == 0 && counters) {
+    atomicAdd(counters + 0, s_pp);
+    atomicAdd(counters + 1, s_rays);
+  }
+}
+
 template <bool OCC, int QB>
 __global__ void __launch_bounds__(256, RVF_FAST_MIN_BLOCKS) k_fast_mixed(const MixedArgs a, unsigned long long* task_ctr,
                                                                         unsigned long long* counters) {
@@ -1317,6 +1340,11 @@ cudaError_t preload_fast() {
   touch((const void*)k_fast_fp64<true, false, Q>);    \
   touch((const void*)k_fast_fp64<false, true, Q>);    \
   touch((const void*)k_fast_fp64<false, false, Q>);
+#define RVF_TOUCH_FLAT(Q)                       \
+  touch((const void*)k_fast_flat<true, Q>);      \
+  touch((const void*)k_fast_flat<false, Q>);
+  RVF_TOUCH_FLAT(3) RVF_TOUCH_FLAT(4) RVF_TOUCH_FLAT(7)
+#undef RVF_TOUCH_FLAT
   RVF_TOUCH_MIXED(2) RVF_TOUCH_MIXED(3) RVF_TOUCH_MIXED(4) RVF_TOUCH_MIXED(5) RVF_TOUCH_MIXED(7) RVF_TOUCH_MIXED(8)
   RVF_TOUCH_FP64(2) RVF_TOUCH_FP64(3) RVF_TOUCH_FP64(4)
 #undef RVF_TOUCH_MIXED
@@ -1326,9 +1354,11 @@ cudaError_t preload_fast() {
 
 cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs& a, const MixedArgs& m,
                         unsigned long long* task_ctr, unsigned long long* counters, int sm_count, cudaStream_t st) {
+  // FP64 surfaces with rules of up to seven points, tasks of whole warps' rows: plane pairs row set by row set
+  const bool flat = !mixed && dim3 && a.pmax <= kFlatPoints && a.fast_groups <= 8;
   auto launch = [&](auto fn, const auto& args) -> cudaError_t {
     int per_sm = 1;
-    const size_t smem = stage_bytes(mixed ? m.pmax : a.pmax);
+    const size_t smem = stage_bytes(mixed ? m.pmax : a.pmax) * (flat ? kFlatRows : 1);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
     fn<<<(unsigned)(sm_count * per_sm), 256, smem, st>>>(args, task_ctr, counters);
     return cudaGetLastError();
@@ -1343,6 +1373,11 @@ cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs&
       case 8: return occ ? launch(k_fast_mixed<true, 8>, m) : launch(k_fast_mixed<false, 8>, m);
       default: return cudaErrorInvalidValue;
     }
+  }
+  if (flat && fast_qb_supported(false, qb)) {
+    if (a.pmax <= 3) return occ ? launch(k_fast_flat<true, 3>, a) : launch(k_fast_flat<false, 3>, a);
+    if (a.pmax == 4) return occ ? launch(k_fast_flat<true, 4>, a) : launch(k_fast_flat<false, 4>, a);
+    return occ ? launch(k_fast_flat<true, 7>, a) : launch(k_fast_flat<false, 7>, a);
   }
   switch (qb) {
 #define RVF_FAST64(Q)                                                                          \
