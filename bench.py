@@ -50,11 +50,11 @@ REF_COUNTS = {
     "full": {"n_rays": 38102400000, "node_visits": 222278703194, "prim_tests": 142516108216},
 }
 # DRAM bytes per traced ray of the traversal phase, pair lists included
-# (dram__bytes_read.sum + dram__bytes_write.sum of k_trace32 / k_trace64 and
-# k_plist in one ncu capture of the medium workload divided by the rays it
-# traced; the capture is summarized under profiles/).
-TRAFFIC_PER_TRACED_RAY = {"mixed": (0.987216e9 + 0.019866e9 + 0.039880e9 + 0.225654e9) / 75262173,
-                          "fp64": (0.990203e9 + 0.017742e9 + 0.039880e9 + 0.225654e9) / 75267549}
+# (dram__bytes_read.sum + dram__bytes_write.sum of k_occ_list and k_occ_pairs in
+# one ncu capture of the medium workload divided by the rays it traced; the
+# capture is summarized under profiles/).
+TRAFFIC_PER_TRACED_RAY = {"mixed": (0.000723e9 + 0.051740e9 + 0.106737e9 + 0.024593e9) / 75262169,
+                          "fp64": (0.000657e9 + 0.026344e9 + 0.080724e9 + 0.013040e9) / 36323189}
 
 
 def load_pkg():
@@ -333,7 +333,7 @@ def roof_for(W: Workload, stats, prec, size, peak64, peak32):
         achieved = flops / (ms / 1e3) / 1e12
         return {"bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": "measured by rvf_fma_peak (FMA microbenchmark) in this run",
-                "kernel": "k_pairs_mc<DIM3=0,OCC=1> (+ k_mc_area)", "kernel_ms_per_launch": ms,
+                "kernel": "k_mc_curves<OCC=1> (+ k_mc_area)", "kernel_ms_per_launch": ms,
                 "launches_per_step": 1, "algorithmic_flop_per_launch": flops,
                 "work_counts": "sample pairs, box and segment tests as executed"}
     if not W.obs:
@@ -342,10 +342,10 @@ def roof_for(W: Workload, stats, prec, size, peak64, peak32):
         achieved = flops / (ms / 1e3) / 1e12
         return {"bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": "measured by rvf_fma_peak (FMA microbenchmark) in this run",
-                "kernel": "k_gen_mixed<OCC=0>" if prec == "mixed" else "k_gen_fp64<DIM3=1,OCC=0>",
+                "kernel": "k_fast_mixed<OCC=0> (+ k_gen_mixed)" if prec == "mixed" else "k_fast_fp64<DIM3=1,OCC=0>",
                 "kernel_ms_per_launch": ms, "launches_per_step": 1, "algorithmic_flop_per_launch": flops,
                 "work_counts": "23 flop per quadrature point pair (Duffy pairs run in k_duffy, timed in phases)"}
-    kernel = "k_plist + k_trace32 (+ k_trace64 re-traversal)" if prec == "mixed" else "k_plist + k_trace64<DIM3=1>"
+    kernel = "k_occ_list + k_occ_pairs<MIXED=%d>" % (prec == "mixed")
     return roofline(stats, peak, bound, kernel, prec, size)
 
 

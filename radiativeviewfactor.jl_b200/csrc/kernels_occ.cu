@@ -24,17 +24,25 @@
 // usable list, or with an infinite 1/d, walks the tree.
 //
 // Measured on a B200, closed cube of 43,200 Tri3 with a box of 1,728 triangles,
-// 7 points (FP64 / mixed precision, one solve): lists 41 / 41 ms, rest 22 / 16
-// ms, pairs 97 / 131 ms, 160 / 188 ms together, bound by instruction issue
-// (65-75% of the slots).  The queue pipeline (kernels_wave.cu), which also needs
-// the classification's pair masks (36 ms), took 310 / 224 ms for the same
-// tiles: a record per ray and a slot and list per pair through global memory,
-// read back with dependent loads at 12 to 15 of 32 active lanes.
+// 7 points (FP64 / mixed precision, one solve): lists 41 / 42 ms, rest 13 / 16
+// ms, pairs 90 / 105 ms, 144 / 163 ms together, bound by instruction issue
+// (65-75% of the slots).  Of the pairs' time about 24 / 30 ms set the rays up,
+// 58 ms test lists, the rest tests uncertain rays again.  The queue pipeline
+// (kernels_wave.cu), which also needs the classification's pair masks (36 ms), took
+// 310 / 224 ms for the same tiles: a record per ray and a slot and list per pair
+// through global memory, read back with dependent loads at 12 to 15 of 32 active
+// lanes.
 // Measured and not kept: all three steps in one kernel, lane = (pair, q) (284 /
 // 311 ms: 16 warps per SM cannot hide the list building's latency, four pairs'
 // lists differ in length); the (ray, triangle) tests packed into full warps
 // through shared memory (144 / 190 ms of pair kernel); the passing rays of a
-// leaf packed into the first lanes (111 / 158 ms).
+// leaf packed into the first lanes (111 / 158 ms); a leaf's triangles before its box
+// (131 / 150 ms against 95 / 112 then: the box stops most warps); the next entry's
+// box or triangle loaded ahead (within 1%, up to 3% slower); a second culling of
+// the lists by the points' extent across the pair's direction (18% fewer list pairs,
+// lists +8 / +15 ms, pairs -14 / -8 ms; mixed precision must keep the sums of the
+// capsule's lists); a lane per pair in the list tests where many pairs reach a leaf
+// (within 1%).
 #include <cuda_runtime.h>
 
 #include <algorithm>

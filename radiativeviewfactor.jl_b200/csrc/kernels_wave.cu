@@ -1,8 +1,12 @@
-// kernels_wave.cu -- the wavefront pair pipeline with occlusion.
+// kernels_wave.cu -- the queue pipeline, and the quadrature-only tiles' kernels.
 //
 // Replaces _vf_pair_kernel! (src/GPUKernels.jl:226-323) with its shadow rays
-// (src/GPUKernels.jl:289-304, gpu_intersect_bvh src/GPUBVH.jl:202-285) when
-// the mesh has obstructions.  One chunk of the upper-triangle tiles runs as
+// (src/GPUKernels.jl:289-304, gpu_intersect_bvh src/GPUBVH.jl:202-285).  Tiles
+// with ray work run here when the occlusion kernels (kernels_occ.cu,
+// kernels_occ2d.cu) do not take them: solves with a ray log (every ray's decision
+// in a record), without tile classification, and obstructions beyond the lists'
+// index widths; and the listed tiles (near field) of mixed-precision solves without
+// obstruction.  One chunk of the upper-triangle tiles runs as
 //   1. generation: the quadrature of every pair (tile-staged as in the fused
 //      kernel).  A ray that misses the root box is visible and its term is
 //      summed at once; every other ray is appended to a global ray queue as
