@@ -22,7 +22,7 @@ struct SegScene {
 };
 
 constexpr int kSegs = 2048;  // segments of a tile's list
-constexpr int kRowItems = 1024;  // (pair, segment) items of a row's pairs (more: its rays walk the tree)
+constexpr int kRowItems = 2048;  // (pair, segment) items of a row's pairs (more: its rays walk the tree)
 constexpr int kFront = kTileFront;
 
 struct SegTile {

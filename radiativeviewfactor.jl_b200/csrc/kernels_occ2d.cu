@@ -19,7 +19,11 @@
 // obstruction, nquad 4: 4.2 ms a solve; walking the tree for every ray took
 // 47 ms (39 segment and 16 box tests a ray, from shared memory at 79% of its
 // bandwidth), a lane testing its own pair's list 4.8 ms (lists differ in length
-// between the lanes).  Bound by FP64 issue.
+// between the lanes).  Bound by issue: a row's set-up weighs against 16 point pairs.
+// Coarse walls (4 elements a side) around four circles of 60, nquad 8, every row
+// walking: 1.26 ms with the row's rays walking together and 2,048 tests a row, 3.5 ms
+// with a walk per lane and 1,024; 1.1 ms in the queue pipeline, which spreads 256
+// elements' rays over the chip (others of these sizes: 0.3-0.9 against 0.8-1.1 ms).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -31,13 +35,14 @@ namespace rvf {
 
 __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ Lp) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ SegTile T;
+  SegTile& T = *reinterpret_cast<SegTile*>(smem);
   const OccBatch& B = *Lp;
   __shared__ int64_t s_tile;
   __shared__ int s_req, s_part, s_row, s_segs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* S = reinterpret_cast<double*>(smem) + warp * 8 * B.pmax_max;
-  uint32_t n_pp = 0, n_rays = 0, n_nodes = 0, n_prims = 0, n_traced = 0;
+  double* S = reinterpret_cast<double*>(smem + sizeof(SegTile)) + warp * 8 * B.pmax_max;
+  uint32_t n_pp = 0, n_rays = 0, n_traced = 0;
+  TravCount tc;
   for (;;) {
     if (threadIdx.x == 0) {
       const unsigned long long k = atomicAdd(B.q.ctr + kCtrTile, 1ull);
@@ -114,6 +119,7 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
       n_pp += (uint32_t)(npi * npj);
       const double* jb = t.tab + bj * kComp * pm * kTile + lane;
       const int qmax = __reduce_max_sync(kFull, npj);
+      const int32_t g_i = t.group[i];
       double acc = 0.0;  // twice the pair's sum
       for (int q = 0; q < qmax; ++q) {
         const bool lq = q < npj;
@@ -141,26 +147,20 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
           const double to[2] = {sw ? xi[0] : xj[0], sw ? xi[1] : xj[1]};
           bool blocked = false;
           if (n > 0) {
-            blocked = (items_block(sc, T, warp, n, casts, from, to, n_nodes, n_prims) >> lane) & 1u;
-          } else if (cast) {
+            blocked = (items_block(sc, T, warp, n, casts, from, to, tc.nodes, tc.prims) >> lane) & 1u;
+          } else {  // the row's rays walk the tree together
             const double lx = fmin(from[0], to[0]), hx = fmax(from[0], to[0]);
             const double ly = fmin(from[1], to[1]), hy = fmax(from[1], to[1]);
-            const int32_t g_i = t.group[i];
-            for (int k = 0; k < t.n_nodes && !blocked;) {  // miss links point forward
-              const NodeD nd = t.nodes[k];
-              ++n_nodes;
-              if (nd.lo[0] > hx || nd.hi[0] < lx || nd.lo[1] > hy || nd.hi[1] < ly) {
-                k = nd.miss;
-                continue;
-              }
-              for (int u = nd.a; u < nd.a + nd.b && !blocked; ++u) {
-                const SegD sg = t.segs[u];
-                if (sg.group == g_i || sg.group == gj) continue;
-                ++n_prims;
-                blocked = seg_blocks(sg, from, to);
-              }
-              k = nd.b > 0 ? nd.miss : k + 1;
-            }
+            blocked = packet_any_hit(
+                cast, t.nodes, t.n_nodes,
+                [&](const NodeD& nd) { return !(nd.lo[0] > hx || nd.hi[0] < lx || nd.lo[1] > hy || nd.hi[1] < ly); },
+                [&](int u, bool test) {
+                  const SegD sg = t.segs[u];
+                  if (!test || sg.group == g_i || sg.group == gj) return false;
+                  ++tc.prims;
+                  return seg_blocks(sg, from, to);
+                },
+                tc);
           }
           if (cast && !blocked) inner = fma(S[8 * p + 3], k, inner);
         }
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
     __syncthreads();
   }
   if (B.counters) {
-    const uint32_t v[4] = {n_pp, n_rays, n_nodes, n_prims};
+    const uint32_t v[4] = {n_pp, n_rays, tc.nodes, tc.prims};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint64_t s = warp_sum_u64(v[k]);
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
 }
 
 cudaError_t launch_occ2d(int pmax, const OccBatch* b, int sm_count, cudaStream_t st) {
-  const size_t smem = stage_bytes(pmax);
+  const size_t smem = sizeof(SegTile) + stage_bytes(pmax);
   const cudaError_t e = cudaFuncSetAttribute(k_occ2d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k_occ2d<<<(unsigned)(2 * sm_count), 256, smem, st>>>(b);
