@@ -77,6 +77,7 @@ struct TileClassArgs {
   float sat_em;
   uint8_t* cls;    // n_tiles
   uint32_t* mask;  // n_tiles x 32, or null: classes only
+  int parts;       // claims a tile (launch_tile_class)
   unsigned long long* claim;  // zeroed tile counter (warps claim tiles one at a time)
   unsigned long long* counters;  // [culled tiles, masked pairs, tiles left unclassified]
 };

@@ -84,8 +84,11 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
     // tiles claimed one at a time: their costs differ by orders of magnitude
     unsigned long long tc = 0;
     if (lane == 0) tc = atomicAdd(a.claim, 1ull);
-    const int64_t t = (int64_t)__shfl_sync(kFull, tc, 0);
+    tc = __shfl_sync(kFull, tc, 0);
+    const int64_t t = MASK ? (int64_t)(tc / (unsigned)a.parts) : (int64_t)tc;
     if (t >= a.n_tiles) break;
+    // with few tiles a claim is a part of a tile's mask rows (the first part also writes what is the tile's)
+    const int part = MASK ? (int)(tc - (unsigned long long)t * (unsigned)a.parts) : 0;
     int64_t bi, bj;
     tile_coords(t, a.nT, bi, bj);
     const int64_t ei = bi * kTile + lane, ej = bj * kTile + lane;
@@ -245,9 +248,11 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
       n_over += all_ones && lane == 0 ? 1 : 0;
     } else if (all_ones) {
       cls |= kClsSlow;
-      a.mask[t * kTile + lane] = 0xffffffffu;
-      n_masked += 32;
-      n_over += lane == 0 ? 1 : 0;
+      if (part == 0) {
+        a.mask[t * kTile + lane] = 0xffffffffu;
+        n_masked += 32;
+        n_over += lane == 0 ? 1 : 0;
+      }
     } else if (nl > 0) {
       // per pair: some listed triangle survives the pair-list tests.  Row by
       // row, the warp first keeps the runs (leaves with listed triangles)
@@ -255,7 +260,8 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
       // radius max(rad_i, rad_J)) can reach, 32 at a time; each lane then
       // tests its pair against those leaves and their triangles.
       cls |= kClsSlow;
-      for (int li = 0; li < kTile; ++li) {
+      const int rows = kTile / a.parts;
+      for (int li = part * rows; li < (part + 1) * rows; ++li) {
         const int64_t i = bi * kTile + li;
         const double x0 = __shfl_sync(kFull, ci[0], li), x1 = __shfl_sync(kFull, ci[1], li),
                      x2 = __shfl_sync(kFull, ci[2], li);
@@ -358,9 +364,9 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
         }
       }
     } else if (a.occ) {
-      ++n_culled;
+      n_culled += part == 0 ? 1 : 0;
     }
-    if (lane == 0) a.cls[t] = cls;
+    if (lane == 0 && part == 0) a.cls[t] = cls;
   }
   if (a.counters) {
     const uint64_t s_c = warp_sum_u64(lane == 0 ? n_culled : 0), s_m = warp_sum_u64(n_masked),
@@ -373,14 +379,20 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
   }
 }
 
-cudaError_t launch_tile_class(const TileClassArgs& a, int sm_count, cudaStream_t st) {
-  if (a.n_tiles <= 0) return cudaSuccess;
+cudaError_t launch_tile_class(const TileClassArgs& args, int sm_count, cudaStream_t st) {
+  if (args.n_tiles <= 0) return cudaSuccess;
+  TileClassArgs a = args;
+  a.parts = 1;
   auto launch = [&](auto fn) -> cudaError_t {
     int per_sm = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kCullWarps * 32, 0) != cudaSuccess || per_sm < 1)
       per_sm = 1;
-    const int64_t want = (a.n_tiles + kCullWarps - 1) / kCullWarps;
-    const int grid = (int)std::min<int64_t>(want, (int64_t)sm_count * per_sm);
+    const int64_t resident = (int64_t)sm_count * per_sm;
+    // masks: four claims a warp, so that the heaviest tiles do not end alone (2,346 tiles of
+    // Monte Carlo masks around a box: 2.9 ms with whole tiles, 1.6 ms with parts of them)
+    while (a.mask && a.parts < 8 && a.n_tiles * a.parts < 4 * kCullWarps * resident) a.parts *= 2;
+    const int64_t want = (a.n_tiles * a.parts + kCullWarps - 1) / kCullWarps;
+    const int grid = (int)std::min<int64_t>(want, resident);
     const cudaError_t e = cudaMemsetAsync(a.claim, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     fn<<<(unsigned)grid, kCullWarps * 32, 0, st>>>(a);

@@ -24,7 +24,7 @@
 // take one division and a corrected product each (div_by).
 //
 // Measured on a B200, 64 samples a pair.  Closed cube of 2,166 Quad4 with a box:
-// rows 4.4 ms, blockable pairs (7% of all) 5.2 ms, classification 2.9 ms; one kernel
+// rows 4.4 ms, blockable pairs (7% of all) 5.0 ms, classification 1.6 ms; one kernel
 // with a tree walk in every masked row took 46 ms (2.6 of a row's 32 pairs masked,
 // eight warps at a barrier per tile).  Rows are bound by FP64 issue (66% of the
 // pipe), blockable pairs by the walks' issue and latency.  Cavity of 4,000 Line3 with
