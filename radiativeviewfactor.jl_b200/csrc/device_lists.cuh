@@ -11,22 +11,32 @@ namespace rvf {
 
 // True when no ray of the pair (segments within R of the centroid segment
 // a -> a + d) can be a hit of the reference's test of the triangle
-// with corners p0, p1, p2 (FP32) and rounding margin p0.w.  em absorbs the
-// FP32 rounding of the corners and of this test (a few 2^-24 of the
-// coordinates' magnitude, against em = S 2^-16).
-__device__ __forceinline__ bool pair_misses_tri(const float* a, const float* d, float R, float em, const float4& p0,
-                                                const float4& p1, const float4& p2) {
+// with corners p0, p1, p2 (FP32) and rounding margin p0.w.  em = S 2^-16 (S: at least
+// |d| and every edge) absorbs the FP32 rounding of the corners and of the
+// projections (a few 2^-24 S |w|).
+//
+// An axis w = d x f of an edge f is taken to see the segment as the point 0 and the
+// edge as one point, so that two corners' projections decide.  The computed w
+// misses both directions by its own rounding, which does not shrink with |w| when
+// f is nearly parallel to d: with u = 2^-24, |w - d x f| <= 2.5 u |d| |f|, and f is
+// rounded by u |f|, so the segment spans up to 2.5 u |d|^2 |f| and the edge up to
+// 3.5 u |d| |f|^2, together at most 6 u S |d| |f| = (6/256) em |d| |f|.  The gap is
+// taken smaller by em/32 |d|_1 |f|_1.  The normal likewise: f1.n and f2.n are at most
+// 3.5 u |f1| |f2| max(|f1|, |f2|).  (Without this, triangles with an edge along the pair's
+// direction, and slivers, lost up to 16% of those a ray of the pair does hit.)
+__host__ __device__ __forceinline__ bool pair_misses_tri(const float* a, const float* d, float R, float em,
+                                                         const float4& p0, const float4& p1, const float4& p2) {
   const float rm = R + p0.w + em, rm2 = rm * rm;
   const float s0[3] = {p0.x - a[0], p0.y - a[1], p0.z - a[2]};
   const float s1[3] = {p1.x - a[0], p1.y - a[1], p1.z - a[2]};
   const float s2[3] = {p2.x - a[0], p2.y - a[1], p2.z - a[2]};
-  // w = d x (edge g - e): the whole segment projects onto 0 (from a), both ends
-  // of the edge onto g.w, the third corner onto h.w
+  const float c = -0.03125f * em, cd = c * (fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]));
+  // w = d x (edge g - e): the segment at 0 (from a), the edge at g.w, the third corner at h.w
   auto edge = [&](const float4& e, const float4& g, const float* sg, const float* sh) {
     const float fx = g.x - e.x, fy = g.y - e.y, fz = g.z - e.z;
     const float wx = d[1] * fz - d[2] * fy, wy = d[2] * fx - d[0] * fz, wz = d[0] * fy - d[1] * fx;
     const float u = fmaf(sg[0], wx, fmaf(sg[1], wy, sg[2] * wz)), v = fmaf(sh[0], wx, fmaf(sh[1], wy, sh[2] * wz));
-    const float gap = fmaxf(fminf(u, v), -fmaxf(u, v));
+    const float gap = fmaf(cd, fabsf(fx) + fabsf(fy) + fabsf(fz), fmaxf(fminf(u, v), -fmaxf(u, v)));
     return gap > 0.0f && gap * gap > rm2 * fmaf(wx, wx, fmaf(wy, wy, wz * wz));
   };
   if (edge(p0, p1, s0, s2)) return true;
@@ -36,7 +46,8 @@ __device__ __forceinline__ bool pair_misses_tri(const float* a, const float* d, 
   const float f1[3] = {p1.x - p0.x, p1.y - p0.y, p1.z - p0.z}, f2[3] = {p2.x - p0.x, p2.y - p0.y, p2.z - p0.z};
   const float nx = f1[1] * f2[2] - f1[2] * f2[1], ny = f1[2] * f2[0] - f1[0] * f2[2], nz = f1[0] * f2[1] - f1[1] * f2[0];
   const float u = fmaf(s0[0], nx, fmaf(s0[1], ny, s0[2] * nz)), e = fmaf(d[0], nx, fmaf(d[1], ny, d[2] * nz));
-  const float gap = fmaxf(u - fmaxf(e, 0.0f), fminf(e, 0.0f) - u);
+  const float gap = fmaf(c * (fabsf(f1[0]) + fabsf(f1[1]) + fabsf(f1[2])), fabsf(f2[0]) + fabsf(f2[1]) + fabsf(f2[2]),
+                         fmaxf(u - fmaxf(e, 0.0f), fminf(e, 0.0f) - u));
   return gap > 0.0f && gap * gap > rm2 * fmaf(nx, nx, fmaf(ny, ny, nz * nz));
 }
 
