@@ -84,11 +84,18 @@ __device__ __forceinline__ int slab_f(const NodeF& nd, const RayF& R) {
 struct MtTol {
   float e0, d;
 };
+// kMtLoose: rays formed in FP32 as r = (c_j - c_i) + (o_q - o_p), with
+// Q = |c_j - c_i| + rad_i + rad_j at most 33 |r| (kMinRay2; shorter ones go to FP64:
+// elements can bulge far beyond their corners).  With u = 2^-24 and
+// |c_j - c_i| + |o_p| + |o_q| <= Q, |o_q - o_p| <= Q + |r|, the direction is off by at
+// most u (2 Q + 2 |r|) / |r| + 5 u <= 73 u in each component, so the largest of the
+// terms below, a, by 1.73 (1.41 74 + 2) u n1 n2 = 184 u n1 n2, against 256 u.
 constexpr MtTol kMtLoose{kE0, 2.0f};
+constexpr float kMinRay2 = 1.0f / 1089.0f;  // |r|^2 / Q^2
 // For rays whose direction is off by at most 7 2^-24 in each component: r formed
-// in FP64 and rounded, or as (c_j - c_i) + (o_q - o_p) in FP32 with the centroids
-// at least two diameters apart (|r| >= 0.4 |c_j - c_i|, |o| <= 0.6 diameters:
-// 2^-24 (2.5 + 3 + 1), and the scaling's rounding).  With u = 2^-24, ns = |s|_1:
+// in FP64 and rounded, or as above with |o_p| + |o_q| <= 0.6 D, D = |c_j - c_i|, so that
+// |r| >= 0.4 D:
+// 2^-24 (2.5 + 3 + 1), and the scaling's rounding.  With u = 2^-24, ns = |s|_1:
 // h = d x e2 is within 13.4 u n2 a component, so U = s.h within
 // (13.4 + 3 + 1) u ns n2 = 2^-19.9 ns n2, V within (1.73 4.5 + 12 + 5) u ns n1 =
 // 2^-19.4 ns n1, T within 14.5 u ns n1 n2 and a within 30 u n1 n2 = 2^-19.1 n1 n2:

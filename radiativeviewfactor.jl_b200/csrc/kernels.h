@@ -357,6 +357,7 @@ enum : int {
   kOccSame = 1 << 8,   // the elements share one normal
   kOccNear = 1 << 9,   // near field (mixed precision)
   kOccOut = 1 << 10,   // every ray misses the root box (mixed precision)
+  kOccTight = 1 << 11, // the rays' directions meet kMtTight's bound (mixed precision)
 };
 struct OccSlot {
   int32_t i, j, req, n;  // req: the request, with the pair's flags above its low byte

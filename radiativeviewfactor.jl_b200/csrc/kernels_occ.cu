@@ -625,8 +625,10 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
           flags |= kOccSame;
         if (t.mixed) {
           const double d0 = cj[0] - t.cen[3 * i], d1 = cj[1] - t.cen[3 * i + 1], d2 = cj[2] - t.cen[3 * i + 2];
-          const double dm = fmax(t.diam[i], t.diam[j]) * t.near_factor;
-          if (d0 * d0 + d1 * d1 + d2 * d2 < dm * dm) flags |= kOccNear;
+          const double dm = fmax(t.diam[i], t.diam[j]) * t.near_factor, dd = d0 * d0 + d1 * d1 + d2 * d2;
+          const double sr = t.rad[i] + rj;
+          if (dd < dm * dm) flags |= kOccNear | kOccTight;  // (near: rays formed in FP64)
+          else if (sr * sr <= 0.36 * dd) flags |= kOccTight;
           if (pair_misses_box<true>(t.cen + 3 * i, cj, fmax(t.rad[i], rj) + t.cull_margin, t.nodes[0]))
             flags |= kOccOut;
         }
@@ -846,7 +848,7 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
       const NodeF* nodesf = t.nodesf;
       const TriF* trisf = t.trisf;
       const float delta = t.delta;
-      const MtTol tol = !MIXED || t.near_factor >= 2.0 ? kMtTight : kMtLoose;
+      const MtTol tol = !MIXED || (ps.req & kOccTight) ? kMtTight : kMtLoose;
       const double* it = t.tab + tab_at(i, 0, 0, pm);
       const double* jt = t.tab + tab_at(j, 0, 0, pm);
       const float per = 1.0f / (float)pm;  // v + 1/2 is at least 1/128 from a multiple of pm, v < 448
@@ -869,11 +871,16 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
       }
       double ci[3], dc[3];
       bool near = false, cullp = false;
+      float r2_min = 1e-18f;  // shorter far rays go to FP64 (kMtLoose)
       if constexpr (MIXED) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           ci[k] = t.cen[3 * i + k];
           dc[k] = t.cen[3 * j + k] - ci[k];
+        }
+        if (!(ps.req & kOccTight)) {
+          const double span = sqrt(dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2]) + t.rad[i] + t.rad[j];
+          r2_min = fmaxf(r2_min, kMinRay2 * (float)(span * span));
         }
         near = (ps.req & kOccNear) != 0;
         n_near += near && npj > 0 && lane == 0 ? 1 : 0;
@@ -976,7 +983,7 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
           }
           n_rays += cast ? 1 : 0;
           if (cast && !cullp) {
-            const bool rok = r2 > 1e-18f && (sw ? make_ray_f(xo, -rx, -ry, -rz, r2, delta, R[u])
+            const bool rok = r2 > (exact ? 1e-18f : r2_min) && (sw ? make_ray_f(xo, -rx, -ry, -rz, r2, delta, R[u])
                                                 : make_ray_f(xo, rx, ry, rz, r2, delta, R[u]));
             if (rok) {
               const int sr = slab_f(nodesf[0], R[u]);

@@ -565,6 +565,8 @@ __global__ void __launch_bounds__(256, 2) k_gen_mixed(const GenBatch* __restrict
       }
       n_near += (near && npj > 0) ? 1 : 0;
       const float d0 = (float)dc0, d1 = (float)dc1, d2 = (float)dc2;
+      const double span = sqrt(dc0 * dc0 + dc1 * dc1 + dc2 * dc2) + (OCC && valid && a.rad ? a.rad[i] + a.rad[j] : 0.0);
+      const float r2_min = kMinRay2 * (float)(span * span);  // shorter rays go to FP64 (kMtLoose)
       // FP32 ray origin anchor: the centroid of the casting element
       const float an0 = (float)(ci0 + (sw ? dc0 : 0.0)), an1 = (float)(ci1 + (sw ? dc1 : 0.0)),
                   an2 = (float)(ci2 + (sw ? dc2 : 0.0));
@@ -614,8 +616,8 @@ __global__ void __launch_bounds__(256, 2) k_gen_mixed(const GenBatch* __restrict
           } else if (OCC && cast32) {
             RayF R;
             const float xo[3] = {an0 + (sw ? oq0 : op0), an1 + (sw ? oq1 : op1), an2 + (sw ? oq2 : op2)};
-            const bool rok =
-                sw ? make_ray_f(xo, -rx, -ry, -rz, r2, a.delta, R) : make_ray_f(xo, rx, ry, rz, r2, a.delta, R);
+            const bool rok = r2 > r2_min && (sw ? make_ray_f(xo, -rx, -ry, -rz, r2, a.delta, R)
+                                                : make_ray_f(xo, rx, ry, rz, r2, a.delta, R));
             badray = !rok;
             if (rok) {
               defer32 = slab_f(s_rootf, R) != kMiss;
