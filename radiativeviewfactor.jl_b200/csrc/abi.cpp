@@ -324,6 +324,7 @@ int mesh_upload(Session* s, const rvf_mesh_desc* d, rvf_mesh** out) {
       mx = std::max(mx, std::fabs(d->coords[k]));
     }
     m->extent = 1.0 + mx;
+    m->max_coord = mx;
   }
 
   // obstruction BVH (exact tree of src/BVH.jl over the merged soup)

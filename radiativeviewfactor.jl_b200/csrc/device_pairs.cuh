@@ -100,8 +100,12 @@ __device__ __forceinline__ void fma_if_facing(double& s, double w, double k, int
 // points -- so a point pair costs r, r^2, 1 / r^4 and one multiply-add, 11
 // FP64 instructions instead of 19, and no sign or grazing test.  A pair with a
 // |cos| below 1e-3 (d^2 <= limit for some d; limit = 1e-6 of the largest
-// possible r^2) is left to the general loop: its cosines would lose more than
-// three digits to the points' rounding.
+// possible r^2), or a point within 1e-4 M of the other element's plane (M: the
+// mesh's largest coordinate), is left to the general loop.  A point of an element is
+// rounded by up to 10 2^-53 M along the normal, for which the d of one point and of
+// another differ: by 1.2e-11 of d at 1e-4 M, 2.4e-11 in the product of two, against the
+// written 1e-10.  Cube of 588 Tri3 1e4 / 1e5 from the origin: off by 2.3e-12 /
+// 1.3e-15, by 3.5e-11 / 3.5e-10 without the second bound.
 struct FlatSum {
   double sum;  // pi times the pair's sum
   uint32_t cast;
@@ -282,7 +286,7 @@ __device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const doub
     if constexpr (PLANE) {
       const int npf = npj > 0 && a.flat[i] && a.flat[j] && d2 > 64.0 * s2 ? npj : 0;
       if (__any_sync(kFull, npf > 0)) {
-        const FlatSum f = flat_fp64(S, jb, pm, npi, npf, 1.27e-6 * d2);
+        const FlatSum f = flat_fp64(S, jb, pm, npi, npf, fmax(1.27e-6 * d2, a.plane_dist2));
         if (f.done) {
           acc = -f.sum;
           if (OCC) n_rays += f.cast;
@@ -421,7 +425,7 @@ __device__ __forceinline__ void flat_rows(const PairArgs& a, const double* iblk,
       bool ok = valid && flat_i && flat_j && npj > 0 && !same && d2 > 64.0 * (s * s);
       if (__any_sync(kFull, ok)) {
         const int npi = a.np[i];
-        const double limit = 1.27e-6 * d2;
+        const double limit = fmax(1.27e-6 * d2, a.plane_dist2);
         double inner[QB];
 #pragma unroll
         for (int u = 0; u < QB; ++u) inner[u] = 0.0;

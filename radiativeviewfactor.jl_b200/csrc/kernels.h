@@ -135,6 +135,7 @@ struct PairArgs {
   const double* cen;    // pair culling: element centroids and point radii (or null)
   const double* rad;
   double cull_margin;
+  double plane_dist2;  // least squared distance of a point from the other element's plane in flat_fp64
   double* F;        // N x N column-major, caller's element order
   // occlusion (n_nodes == 0: none)
   const NodeD* nodes;

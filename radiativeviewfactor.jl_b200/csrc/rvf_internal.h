@@ -164,6 +164,7 @@ struct rvf_mesh {
   int n_frontier = 0;
   float sat_em = 0.f;
   double extent = 1.0;                        // 1 + max |coordinate| of the mesh and the soup
+  double max_coord = 0.0;                     // max |coordinate| of the mesh's nodes
   int n_nodes = 0;
   int64_t n_obs = 0;
   std::map<int, std::unique_ptr<rvf::Tables>> tables;

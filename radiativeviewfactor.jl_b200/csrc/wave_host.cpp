@@ -142,6 +142,7 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   a.cen = T->cen.as<double>();
   a.rad = T->rad.as<double>();
   a.cull_margin = std::ldexp(m->extent, -30);
+  a.plane_dist2 = 1e-8 * m->max_coord * m->max_coord;
   a.F = m->F.as<double>();
   a.nodes = occ ? m->nodes.as<NodeD>() : nullptr;
   a.n_nodes = occ ? m->n_nodes : 0;
