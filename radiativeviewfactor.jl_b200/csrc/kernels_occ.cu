@@ -399,9 +399,12 @@ __global__ void __launch_bounds__(256, 3) k_occ_list(const OccBatch* __restrict_
       // a tile needs at most 1,024 queue slots; the launch's blocks may each hold one more tile
       const unsigned long long used = *(volatile unsigned long long*)(Q.ctr + kCtrSlots) +
                                       *(volatile unsigned long long*)(Q.ctr + kCtrWalk),
-                               pool = *(volatile unsigned long long*)(Q.ctr + kCtrPool);
+                               pool = *(volatile unsigned long long*)(Q.ctr + kCtrPool),
+                               next = *(volatile unsigned long long*)(Q.ctr + kCtrTile);
+      // a full pool ends the chunk between tiles, not between a tile's parts (the next chunk would do the first
+      // ones again): a block that claimed a part comes back for the rest; pairs that find the pool full walk
       if (used + (unsigned long long)gridDim.x * kTile * kTile <= (unsigned long long)Q.scap &&
-          pool <= (unsigned long long)Q.pool_cap) {
+          (pool <= (unsigned long long)Q.pool_cap || next % (unsigned)B.groups != 0)) {
         const unsigned long long k = atomicAdd(Q.ctr + kCtrTile, 1ull);
         const int64_t g = (int64_t)(k / (unsigned)B.groups);
         if (g < B.total_tiles) {

@@ -500,7 +500,7 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
     ob.n_req = n;
     ob.pmax_max = sh.pmax_max;
     ob.total_tiles = base[n];
-    // a tile is split into tasks only when the queue holds every tile at once
+    // a tile is split into parts only when the queue holds every tile at once: a chunk then ends between tiles
     const bool all = !sh.dim3 || (base[n] + sh.occ_grid) * kTile * kTile <= ob.q.scap;
     ob.groups = all ? occ_groups(base[n], s->sm_count) : 1;
     ob.rest_parts = base[n] * 8 >= (int64_t)64 * s->sm_count ? 8 : 32;
