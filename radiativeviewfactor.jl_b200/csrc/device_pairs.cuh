@@ -356,7 +356,7 @@ __device__ __forceinline__ void gen_fast_fp64_body(const PairArgs& a, const doub
       }
     }
     if (valid) {
-      const double raw = acc * (DIM3 ? -1.0 / kPiD : -0.5);
+      const double raw = fma(acc, DIM3 ? -1.0 / kPiD : -0.5, 0.0);  // (a sum of nothing is +0)
       a.F[oi + oj * N] = raw / a.area[i];
       a.F[oj + oi * N] = raw / a.area[j];
     } else if (j == i) {
