@@ -34,25 +34,26 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return r;
 }
 
-// a / b for several a with one b: y = RN(1 / b) (one division), q0 = RN(a y),
+// a / b for several a with one b > 0: y = RN(1 / b) (one division), q0 = RN(a y),
 // and twice q <- RN(q + RN(a - q b) y).  The first step leaves q0 (off by at
 // most 2 ulp) faithful, after which the second gives RN(a / b) (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
 // 1990: a faithful quotient corrected once by the correctly rounded reciprocal
-// is correctly rounded).  The residuals are exact unless a is so small that
-// they underflow: such a (and b out of the middle range) take the division.
+// is correctly rounded).  Numerators and divisors outside the middle range, where a
+// quotient could overflow or a residual underflow, take the division.  The residual is
+// formed negated: the zero it is for a = -0 then keeps the quotient's sign.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   const double q0 = a * y;
-  const double q1 = fma(fma(-q0, b, a), y, q0);
-  return fma(fma(-q1, b, a), y, q1);
+  const double q1 = fma(-fma(q0, b, -a), y, q0);
+  return fma(-fma(q1, b, -a), y, q1);
 }
-// whether a / b may be taken by div_by: a zero or 2^-700 <= |a| < 2^700 (hi words)
+// whether a / b may be taken by div_by: each a zero or 2^-500 <= |a| < 2^500 (hi words; b not a zero)
 __device__ __forceinline__ bool div_by_ok(double a) {
   const unsigned h = (unsigned)(__double2hiint(a) & 0x7fffffff);
-  return h - 0x14300000u < 0x57800000u || (h | (unsigned)__double2loint(a)) == 0u;
+  return h - 0x20b00000u < 0x3e800000u || (h | (unsigned)__double2loint(a)) == 0u;
 }
 
-// a / b for N values a, each rounded as the division rounds it
+// a / b for N values a and b >= 0, each rounded as the division rounds it (0 / 0: NaN as there)
 template <int N>
 __device__ __forceinline__ void div_all(const double (&a)[N], double b, double (&q)[N]) {
   bool ok = div_by_ok(b);
