@@ -377,7 +377,7 @@ __device__ __forceinline__ double div_or(double a, double b, double y) {
 // is left.  Same sums, bit for bit.  Bound by latency and FP64 issue.  Closed cube of
 // 43,200 Tri3, 7 points, the tiles without ray work: 79 ms with flat_fp64 row by row
 // (stalls on the column's points), 63 ms so.
-constexpr int kFlatRows = kTile / 8, kFlatPoints = 7;
+constexpr int kFlatRows = kTile / 8;
 template <bool OCC, int QB>
 __device__ __forceinline__ void flat_rows(const PairArgs& a, const double* iblk, double* S, int64_t bi, int64_t bj,
                                           int li0, int lane, uint32_t& n_pp, uint32_t& n_rays) {

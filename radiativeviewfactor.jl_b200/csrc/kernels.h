@@ -397,10 +397,17 @@ cudaError_t launch_plist(const TraceBatch* t, int sm_count, cudaStream_t st);
 cudaError_t launch_tile_class(const TileClassArgs& a, int sm_count, cudaStream_t st);
 // Every tile of one request that needs no shadow-ray work (its class), one
 // warp per task (a.fast_groups tasks per tile), before the request's chunks;
-// qb points of the destination element per lane block (fast_qb_default: by
-// the rule's size; fast_qb_supported: the compiled blocks); task_ctr: a
-// zeroed counter.
+// qb points of the destination element per lane block (0: by the rule,
+// fast_flat or fast_qb_default's size; fast_qb_supported: the compiled blocks);
+// task_ctr: a zeroed counter.
 int fast_qb_default(bool mixed, int pmax);
+// Whether the plane pairs run row set by row set (k_fast_flat): FP64 surfaces with
+// rules of up to kFlatPoints points, all held by a lane, in tasks of whole warps'
+// rows, unless the caller names a point block.
+constexpr int kFlatPoints = 7;
+inline bool fast_flat(bool mixed, bool dim3, int pmax, int groups, int qb) {
+  return !mixed && dim3 && pmax <= kFlatPoints && groups <= 8 && qb == 0;
+}
 cudaError_t preload_fast();  // loads every compiled shape (before timing them)
 bool fast_qb_supported(bool mixed, int qb);
 cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs& a, const MixedArgs& m,

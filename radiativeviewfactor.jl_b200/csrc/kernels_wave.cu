@@ -1360,8 +1360,8 @@ cudaError_t preload_fast() {
 
 cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs& a, const MixedArgs& m,
                         unsigned long long* task_ctr, unsigned long long* counters, int sm_count, cudaStream_t st) {
-  // FP64 surfaces with rules of up to seven points, tasks of whole warps' rows: plane pairs row set by row set
-  const bool flat = !mixed && dim3 && a.pmax <= kFlatPoints && a.fast_groups <= 8;
+  const bool flat = fast_flat(mixed, dim3, a.pmax, a.fast_groups, qb);
+  if (qb == 0) qb = fast_qb_default(mixed, mixed ? m.pmax : a.pmax);
   auto launch = [&](auto fn, const auto& args) -> cudaError_t {
     int per_sm = 1;
     const size_t smem = stage_bytes(mixed ? m.pmax : a.pmax) * (flat ? kFlatRows : 1);
@@ -1380,7 +1380,7 @@ cudaError_t launch_fast(bool mixed, bool dim3, bool occ, int qb, const PairArgs&
       default: return cudaErrorInvalidValue;
     }
   }
-  if (flat && fast_qb_supported(false, qb)) {
+  if (flat) {
     if (a.pmax <= 3) return occ ? launch(k_fast_flat<true, 3>, a) : launch(k_fast_flat<false, 3>, a);
     if (a.pmax == 4) return occ ? launch(k_fast_flat<true, 4>, a) : launch(k_fast_flat<false, 4>, a);
     return occ ? launch(k_fast_flat<true, 7>, a) : launch(k_fast_flat<false, 7>, a);

@@ -159,7 +159,7 @@ const int kCand[][2] = {{0, 0}, {2, 0}, {0, 2}, {2, 2}};
 constexpr int kNCand = 4;
 
 // Candidate shapes of the quadrature-only kernel: the default (points by the
-// rule, tasks per tile by the tile count), about half the points per lane
+// rule: 0; tasks per tile by the tile count), about half the points per lane
 // block (fewer registers, more resident warps), and the next finer and the
 // next coarser split of a tile into warp tasks (1, 2, 4, 8, 32).
 constexpr int kNFastCand = 4;
@@ -169,7 +169,7 @@ void fast_cand(bool mixed, int pmax, int64_t n_tiles, int sm_count, size_t c, in
   const int ga = fast_groups_auto(n_tiles, sm_count);
   int k = 0;
   while (steps[k] != ga) ++k;
-  qb = d;
+  qb = 0;
   groups = ga;
   if (c == 1) qb = std::max(2, (d + 1) / 2);
   if (c == 2) groups = steps[k < 4 ? k + 1 : 2];
@@ -895,7 +895,7 @@ int rvf_server_stats_get(rvf_server* sv, rvf_server_stats* st) try {
       o.gen_blocks_per_sm = g->second.gen;
       o.trace_blocks_per_sm = g->second.trace;
     }
-    o.fast_points = f.qb;
+    o.fast_points = f.qb > 0 ? f.qb : fast_qb_default(o.mixed != 0, o.rule_points);
     o.fast_row_groups = f.groups;
     double best = f.score[0];
     for (int c = 1; c < kNFastCand; ++c) best = std::min(best, f.score[c]);

@@ -310,10 +310,9 @@ int wave_fast(Session* s, WaveReq& w, int64_t* n_kernels) {
   w.pa.fast_groups = w.ma.fast_groups =
       w.fast_groups > 0 ? w.fast_groups : fast_groups_auto(w.n_fast_tiles > 0 ? w.n_fast_tiles : w.pa.n_tiles,
                                                            s->sm_count);
-  const int qb = w.fast_qb > 0 ? w.fast_qb : fast_qb_default(w.mixed, w.pmax);
   cudaError_t e = cudaMemsetAsync(s->fast_ctr.ptr, 0, sizeof(unsigned long long), s->stream);
   if (e == cudaSuccess)
-    e = launch_fast(w.mixed, w.dim3, w.occ, qb, w.pa, w.ma, s->fast_ctr.as<unsigned long long>(),
+    e = launch_fast(w.mixed, w.dim3, w.occ, w.fast_qb, w.pa, w.ma, s->fast_ctr.as<unsigned long long>(),
                     s->counters.as<unsigned long long>(), s->sm_count, s->stream);
   if (e != cudaSuccess) return cuda_err(e, "quadrature-only tiles launch");
   if (n_kernels) *n_kernels += 1;
