@@ -268,8 +268,8 @@ typedef struct {
 typedef struct {
   int32_t mixed, occlusion, dim3;
   int32_t size_class;              /* requests with 4^k <= quadrature-only tiles < 4^(k+1) */
-  int32_t gen_blocks_per_sm;       /* chunked generation grid (0: occupancy default; chunk sweep) */
-  int32_t trace_blocks_per_sm;     /* traversal grid (0: occupancy default; chunk sweep) */
+  int32_t gen_blocks_per_sm;       /* queue pipeline's generation grid (0: occupancy default, or not its tiles) */
+  int32_t trace_blocks_per_sm;     /*   and traversal grid */
   int32_t fast_points;             /* quadrature-only kernel: destination points per lane block */
   int32_t fast_row_groups;         /*   and warp tasks per tile */
   int32_t rule_points;             /* quadrature points per element of the class's rule */

@@ -176,9 +176,9 @@ void fast_cand(bool mixed, int pmax, int64_t n_tiles, int sm_count, size_t c, in
   if (c == 3) groups = steps[k > 0 ? k - 1 : 2];
 }
 
-// launch class: precision, surface or curve mesh, occlusion
+// launch class: precision, surface or curve mesh, occlusion, and which kernels its listed tiles run
 uint64_t class_key(const Req* r) {
-  return (uint64_t)r->w.mixed | ((uint64_t)r->w.dim3 << 1) | ((uint64_t)r->w.occ << 2);
+  return (uint64_t)r->w.mixed | ((uint64_t)r->w.dim3 << 1) | ((uint64_t)r->w.occ << 2) | ((uint64_t)r->w.occ_lists << 3);
 }
 
 // launch class and size class (4^k <= quadrature-only tiles < 4^(k+1))
@@ -354,7 +354,8 @@ void run_chunk(rvf_server* sv, std::vector<Req*>& batch) {
   {
     std::lock_guard<std::mutex> lk(s->tune_mu);
     GridTune& t = s->grid_tune[key];
-    if (sv->o.autotune >= 0 && !t.done && batch[0]->w.occ) {
+    // (the occlusion kernels have grids of their own: nothing to choose)
+    if (sv->o.autotune >= 0 && !t.done && batch[0]->w.occ && !batch[0]->w.occ_lists) {
       tuning = true;
       cand = t.next;
       gen = kCand[cand][0];
