@@ -103,7 +103,7 @@ int pmax_of(const rvf_mesh_desc* d, int nquad) {
 // Device memory a request holds from admission to release: F, the
 // quadrature tables (FP64, plus FP32 in mixed mode), per-element arrays,
 // BVH, reductions.
-uint64_t footprint_of(const rvf_mesh_desc* d, const rvf_options* o) {
+uint64_t footprint_of(const rvf_mesh_desc* d, const rvf_options* o, int sm_count) {
   const uint64_t N = (uint64_t)std::max<int64_t>(d->n_elems, 0);
   const uint64_t tiles = (N + kTile - 1) / kTile;
   const uint64_t pm = (uint64_t)pmax_of(d, o->nquad);
@@ -113,7 +113,7 @@ uint64_t footprint_of(const rvf_mesh_desc* d, const rvf_options* o) {
   if (o->precision == RVF_PREC_MIXED) b += tiles * kTile * kComp * pm * 4;  // FP32 table
   b += N * 256 + 24 * (uint64_t)std::max<int64_t>(d->n_nodes, 0);          // per-element arrays, coordinates
   b += (uint64_t)std::max<int64_t>(d->n_obs, 0) * 400;                    // BVH nodes and primitives, both precisions
-  b += (uint64_t)std::min<uint64_t>(256, std::max<uint64_t>(1, (1u << 20) / std::max<uint64_t>(N, 1))) * G * N * 8;
+  b += (uint64_t)reduce_chunks((int64_t)N, sm_count) * G * N * 8;          // reductions' partial sums
   b += (G * N + G * G + G + N) * 8;                                        // row-group, group and row sums
   b += tiles * (tiles + 1) / 2 * (1 + kTile * 4);                          // tile classes and masks
   return b + (1u << 20);
@@ -716,7 +716,7 @@ int rvf_submit(rvf_server* sv, const rvf_mesh_desc* d, const rvf_options* o, int
   r->opts = *o;
   r->n_elems = d->n_elems;
   r->quad = (o->method == RVF_METHOD_QUADRATURE);
-  r->footprint = footprint_of(d, o);
+  r->footprint = footprint_of(d, o, sv->s->sm_count);
   std::lock_guard<std::mutex> lk(sv->mu);
   if (sv->closing) return set_err(RVF_ECLOSED, "server is shutting down");
   r->id = sv->next_id++;
