@@ -52,6 +52,9 @@ enum : uint8_t {
   kClsSlow = 1,  // some pair's rays may be blocked: the ray pipeline, with the mask
   kClsNear = 2,  // some pair is near field (mixed precision integrates it in FP64)
   kClsTiny = 4,  // some pair's points may nearly coincide (mixed precision: FP64)
+  // classes without masks, with kClsSlow: which kernels take the tiles (wave_host.cpp: occ_by_queue)
+  kClsWide = 8,   // the hull reaches more leaves than the walk holds
+  kClsLong = 16,  // or many
 };
 constexpr int kTileLeaves = 256;  // candidate leaves of a tile's walk
 constexpr int kTileFront = 256;   // breadth-first frontier of a tile's walk

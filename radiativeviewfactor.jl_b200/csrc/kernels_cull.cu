@@ -51,6 +51,7 @@ namespace rvf {
 namespace {
 
 constexpr int kCullWarps = 4;
+constexpr int kLongLeaves = 200;  // (about 1,024 triangles)
 
 }  // namespace
 
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
     uint8_t cls = (__any_sync(kFull, near) ? kClsNear : 0) | (__any_sync(kFull, tiny) ? kClsTiny : 0);
     bool all_ones = false;  // occlusion the tile cannot classify: every pair keeps its rays
     int nl = 0;             // listed triangles
+    int n_leaves = 0;       // leaves the hull reaches
     int nrun = 0;           // leaves with listed triangles (runs of the list)
     float rmaxJ = 0.0f;     // largest point radius of the column block
     if (a.occ && !a.dim3) {
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
         nxt = tmp;
         ncur = nnext;
       }
+      n_leaves = nleaf;
       // triangles of the candidate leaves, four leaves of up to 8 per round
       for (int b = 0; b < nleaf && !over; b += 4) {
         const int li = b + (lane >> 3), u8 = lane & 7;
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(kCullWarps * 32, RVF_CULL_MIN_BLOCKS) k_tile_c
       all_ones = over;
     }
     if constexpr (!MASK) {
-      if (all_ones || nl > 0) cls |= kClsSlow;
+      if (all_ones || nl > 0) cls |= kClsSlow | (all_ones ? kClsWide : 0) | (all_ones || n_leaves >= kLongLeaves ? kClsLong : 0);
       else if (a.occ) ++n_culled;
       n_over += all_ones && lane == 0 ? 1 : 0;
     } else if (all_ones) {

@@ -108,6 +108,34 @@ static int ensure_occ(Session* s, int64_t n_tiles, OccQ& q, int& grid) {
   return 0;
 }
 
+// Whether a surface solve's tiles with ray work run in the queue pipeline
+// (kernels_wave.cu) rather than in the occlusion kernels (kernels_occ.cu).  Those
+// build every pair's list from its tile's; where the obstruction is so fine that
+// most tiles reach more leaves or triangles than a tile's list holds, each pair walks
+// the tree itself and, in mixed precision, sums in FP64, which costs more than the
+// rays of a rule of few points.  wide, lng: of the tiles with ray work, the shares
+// beyond the classification's 256 leaves, and with 200 leaves (about 1,024 triangles)
+// or more.  Both sides were measured over 1,232 solves (12 to 30,000 elements of
+// every family, centred boxes of 12 to 10,800 triangles, rules of 1 to 64 points):
+// with lists alone 131 of them were slower than the queue pipeline had been, by up
+// to 1.8x; with these lines 12, by up to 1.07x.  Examples (ms, lists / queue; wide):
+//   FP64, 1 point, 3,750 Quad4, 4,800 triangles (0.94): 8.5 / 4.5; 10,800 Tri3, 2,352 (0.46): 20.2 / 17.4
+//   FP64, 7 points, 1,728 Tri3, 10,800 triangles (0.93): 10.9 / 9.4; 4,800 Tri3, 4,800 (0.81): 41.0 / 47.4
+//   mixed, 13 points, 768 Tri3, 4,800 triangles (1.0): 6.6 / 3.8; 7 points, 30,000 Tri3, 2,352 (0.30): 198 / 232
+//   FP64, 7 points, 108 Tri3, 1,200 triangles (long 1.0): 1.23 / 0.72, the rows of few tiles one after another
+static bool occ_by_queue(bool mixed, bool geometric, int pmax, int64_t n_tiles, double wide, double lng) {
+  const bool few = n_tiles <= 64 && lng >= 0.9 && wide < 0.5;
+  if (pmax == 1 && n_tiles <= 200) return wide >= 0.98;
+  if (pmax <= 4) {
+    if (few && pmax > 1) return true;
+    if (mixed) return n_tiles > 64 && (wide >= (geometric ? 0.15 : 0.25) || lng >= 0.5);
+    return wide >= (geometric ? 0.3 : 0.4);
+  }
+  if (pmax <= 8 && few) return true;
+  if (!mixed) return pmax <= 8 ? wide >= 0.92 : pmax <= 16 && few && n_tiles <= 16;
+  return pmax <= 16 && n_tiles >= 100 && lng >= 0.5;
+}
+
 int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8_t* ray_log, WaveReq& w,
                  int64_t* n_kernels) {
   const int64_t N = m->N;
@@ -236,11 +264,26 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
       if (e2 != cudaSuccess) return cuda_err(e2, "tile classes");
       const uint8_t need = w.mixed ? (uint8_t)(kClsSlow | kClsNear | kClsTiny) : (uint8_t)kClsSlow;
       w.row_end.assign((size_t)a.nT, 0);
-      int64_t t = 0, n_work = 0;
+      int64_t t = 0, n_work = 0, n_slow = 0, n_wide = 0, n_long = 0;
       for (int64_t bi = 0; bi < a.nT; ++bi) {
-        for (int64_t bj = bi; bj < a.nT; ++bj, ++t)
-          if (cls[(size_t)t] & need) work[n_work++] = (int32_t)t;
+        for (int64_t bj = bi; bj < a.nT; ++bj, ++t) {
+          const uint8_t k = cls[(size_t)t];
+          if (k & need) work[n_work++] = (int32_t)t;
+          n_slow += k & kClsSlow ? 1 : 0;
+          n_wide += k & kClsWide ? 1 : 0;
+          n_long += k & kClsLong ? 1 : 0;
+        }
         w.row_end[(size_t)bi] = n_work;
+      }
+      if (w.occ_lists && n_slow > 0 &&
+          occ_by_queue(w.mixed, o->geometric_soup != 0, a.pmax, a.n_tiles, (double)n_wide / n_slow, (double)n_long / n_slow)) {
+        // the queue pipeline, which needs the masks: the same classes again, with them
+        w.occ_lists = false;
+        c.mask = T->tmask.as<uint32_t>();
+        e2 = cudaMemsetAsync(c.counters, 0, 3 * sizeof(unsigned long long), s->stream);
+        if (e2 == cudaSuccess) e2 = launch_tile_class(c, s->sm_count, s->stream);
+        if (e2 != cudaSuccess) return cuda_err(e2, "tile classification launch");
+        if (n_kernels) *n_kernels += 1;
       }
       if (n_work > 0) {
         if (T->twork.bytes < sizeof(int32_t) * n_work && (rc = T->twork.alloc(s, sizeof(int32_t) * n_work))) return rc;
