@@ -148,7 +148,8 @@ __device__ __forceinline__ int tile_segments(const SegScene& sc, const HullF& H,
 // Warp-uniform call and number.
 __device__ __forceinline__ int row_segments(const SegScene& sc, const HullF& H, SegTile& T, int nseg, int warp,
                                             const double* A, const double* cj, double ri, double rj, double rj_max,
-                                            bool valid, bool skip, int32_t gi, int32_t gj, uint32_t& some) {
+                                            bool valid, bool skip, int32_t gi, int32_t gj, uint32_t& some,
+                                            int limit = kRowItems) {
   const int lane = threadIdx.x & 31;
   some = 0;
   int n = 0;
@@ -169,7 +170,7 @@ __device__ __forceinline__ int row_segments(const SegScene& sc, const HullF& H, 
     }
     Hr.c[0][2] = Hr.h[0][2] = Hr.c[1][2] = Hr.h[1][2] = Hr.d[2] = 0.0f;
     const float row_reach = __double2float_ru(fmax(ri, rj_max) + sc.margin) + sc.slack;
-    for (int b = 0; b < nseg; b += 32) {
+    for (int b = 0; b < nseg && n <= limit; b += 32) {
       bool keep = false;
       if (b + lane < nseg) {
         const SegD sg = sc.segs[T.seg[b + lane]];
@@ -191,7 +192,7 @@ __device__ __forceinline__ int row_segments(const SegScene& sc, const HullF& H, 
     }
   }
   __syncwarp();
-  if (nseg < 0 || n > kRowItems) {
+  if (nseg < 0 || n > limit) {
     some = __ballot_sync(kFull, valid);
     return -1;
   }

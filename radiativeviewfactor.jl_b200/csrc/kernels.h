@@ -155,6 +155,7 @@ struct PairArgs {
   int64_t tile0;                 // batched generation: first tile of this request in the launch
   const uint8_t* tcls;           // tile classes and masks (kernels_cull.cu), or null
   const uint32_t* tmask;
+  bool only_masked;              // the masks' pairs alone (the others are integrated elsewhere)
   bool fast_done;                // tiles without ray work were integrated by k_fast_fp64: skip them
   int fast_groups;               // k_fast_fp64 tasks per tile (1, 2 or 4 row groups)
   const int32_t* work;           // the tiles of the chunked pipeline in order (null: every tile)
@@ -355,7 +356,8 @@ struct OccArgs {
   int n_frontier;
   const int32_t* work;
   const uint8_t* tcls;
-  uint32_t* tmask;  // written: the queued pairs of each row of a listed tile
+  uint32_t* tmask;    // written: the queued pairs of each row of a listed tile (curves: the deferred pairs)
+  uint8_t* deferred;  // curves: per tile, kClsSlow when it has deferred pairs
 };
 enum : int {
   kOccSame = 1 << 8,   // the elements share one normal
@@ -387,7 +389,8 @@ struct OccBatch {
   OccQ q;
   unsigned long long* counters;
 };
-// curve meshes with occlusion (kernels_occ2d.cu): every tile, without a queue
+// curve meshes with occlusion (kernels_occ2d.cu): every tile, without a queue; rows beyond its lists are
+// deferred (counted in kCtrWalk) to the queue pipeline
 cudaError_t launch_occ2d(int pmax, const OccBatch* b, int sm_count, cudaStream_t st);
 int occ_groups(int64_t n_tiles, int sm_count);
 int occ_list_grid(int sm_count);  // resident blocks of the list kernel

@@ -13,17 +13,21 @@
 // overlaps the segment's leaf (the leaf box lies in every ancestor's, so the
 // reference's walk reaches it exactly when it does): the decisions are the walk's.
 // A tile with more than kSegs segments within reach, or a row with more than
-// kRowItems tests, walks the tree for every ray.
+// kRowItems tests (half of them in launches of few tiles, whose rows run one
+// after another), is deferred: the queue pipeline (kernels_wave.cu), whose rays
+// walk the tree, takes its pairs after this kernel.
 //
 // Measured on a B200, 2-D cavity of 4,000 Line3 with four circles of 200 as
 // obstruction, nquad 4: 4.2 ms a solve; walking the tree for every ray took
 // 47 ms (39 segment and 16 box tests a ray, from shared memory at 79% of its
 // bandwidth), a lane testing its own pair's list 4.8 ms (lists differ in length
 // between the lanes).  Bound by issue: a row's set-up weighs against 16 point pairs.
-// Coarse walls (4 elements a side) around four circles of 60, nquad 8, every row
-// walking: 1.26 ms with the row's rays walking together and 2,048 tests a row, 3.5 ms
-// with a walk per lane and 1,024; 1.1 ms in the queue pipeline, which spreads 256
-// elements' rays over the chip (others of these sizes: 0.3-0.9 against 0.8-1.1 ms).
+// Fine obstructions, where rows of coarse walls reach thousands of segments (ms,
+// rows beyond the lists walking in this kernel / deferred / all in the queue
+// pipeline): 3,120 Line3 with 3,000 segments, nquad 8, 129 / 14.2 / 29.0; 832 Line3 with
+// 800 segments, nquad 8, 9.8 / 1.9 / 1.5; 2,800 Line3 with 2,000 segments, nquad 3,
+// 3.2 / 3.5 / 12.2.  Limits of 256, 512 and 1,024 tests a row were 14%, 5% and 1% slower
+// over 121 solves.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -41,8 +45,9 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
   __shared__ int s_req, s_part, s_row, s_segs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* S = reinterpret_cast<double*>(smem + sizeof(SegTile)) + warp * 8 * B.pmax_max;
-  uint32_t n_pp = 0, n_rays = 0, n_traced = 0;
+  uint32_t n_pp = 0, n_rays = 0, n_traced = 0, n_defer = 0;
   TravCount tc;
+  const int limit = B.total_tiles <= 64 ? kRowItems / 2 : kRowItems;
   for (;;) {
     if (threadIdx.x == 0) {
       const unsigned long long k = atomicAdd(B.q.ctr + kCtrTile, 1ull);
@@ -104,7 +109,17 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
       // the row's (pair, segment) items, or n = -1 (its rays walk the tree)
       const double A[3] = {t.cen[3 * i], t.cen[3 * i + 1], 0.0};
       uint32_t rest;
-      const int n = row_segments(sc, H, T, nseg, warp, A, cj, t.rad[i], rj, rj_max, valid, true, t.group[i], gj, rest);
+      const int n = row_segments(sc, H, T, nseg, warp, A, cj, t.rad[i], rj, rj_max, valid, true, t.group[i], gj, rest,
+                                 limit);
+      const bool defer = n < 0 && rest != 0;  // warp-uniform
+      if (defer) {
+        if (lane == 0) {  // (zeroed before the launch: a store in every row cost 14% of the kernel)
+          t.deferred[s_tile] = kClsSlow;
+          t.tmask[s_tile * kTile + li] = rest;
+        }
+        ++n_defer;
+        continue;
+      }
       const bool some = (rest >> lane) & 1u;
       fast_fp64<false, true>(a, a.tab + bi * kComp * pm * kTile, S, bi, bj, li + 8, lane, n_pp, n_rays, rest);
       if (rest == 0) continue;  // warp-uniform
@@ -119,7 +134,6 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
       n_pp += (uint32_t)(npi * npj);
       const double* jb = t.tab + bj * kComp * pm * kTile + lane;
       const int qmax = __reduce_max_sync(kFull, npj);
-      const int32_t g_i = t.group[i];
       double acc = 0.0;  // twice the pair's sum
       for (int q = 0; q < qmax; ++q) {
         const bool lq = q < npj;
@@ -145,23 +159,7 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
           // the segment as the reference passes it
           const double from[2] = {sw ? xj[0] : xi[0], sw ? xj[1] : xi[1]};
           const double to[2] = {sw ? xi[0] : xj[0], sw ? xi[1] : xj[1]};
-          bool blocked = false;
-          if (n > 0) {
-            blocked = (items_block(sc, T, warp, n, casts, from, to, tc.nodes, tc.prims) >> lane) & 1u;
-          } else {  // the row's rays walk the tree together
-            const double lx = fmin(from[0], to[0]), hx = fmax(from[0], to[0]);
-            const double ly = fmin(from[1], to[1]), hy = fmax(from[1], to[1]);
-            blocked = packet_any_hit(
-                cast, t.nodes, t.n_nodes,
-                [&](const NodeD& nd) { return !(nd.lo[0] > hx || nd.hi[0] < lx || nd.lo[1] > hy || nd.hi[1] < ly); },
-                [&](int u, bool test) {
-                  const SegD sg = t.segs[u];
-                  if (!test || sg.group == g_i || sg.group == gj) return false;
-                  ++tc.prims;
-                  return seg_blocks(sg, from, to);
-                },
-                tc);
-          }
+          const bool blocked = (items_block(sc, T, warp, n, casts, from, to, tc.nodes, tc.prims) >> lane) & 1u;
           if (cast && !blocked) inner = fma(S[8 * p + 3], k, inner);
         }
         if (lq) acc = fma(jb[(6 * pm + q) * kTile], inner, acc);
@@ -175,6 +173,7 @@ __global__ void __launch_bounds__(256, 2) k_occ2d(const OccBatch* __restrict__ L
     }
     __syncthreads();
   }
+  if (lane == 0 && n_defer) atomicAdd(B.q.ctr + kCtrWalk, (unsigned long long)n_defer);
   if (B.counters) {
     const uint32_t v[4] = {n_pp, n_rays, tc.nodes, tc.prims};
 #pragma unroll

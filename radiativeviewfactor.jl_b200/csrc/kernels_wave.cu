@@ -288,10 +288,10 @@ __global__ void __launch_bounds__(256, 2) k_gen_fp64(const GenBatch* __restrict_
       const int64_t i = bi * kTile + li;
       if (i >= N) continue;  // warp-uniform
       if (a.tcls && !a.ray_log && s_mask[li] == 0u) {  // no ray of this row can be blocked
-        fast_fp64<DIM3, OCC>(a, iblk, S, bi, bj, li + 8, lane, n_pp, n_rays);
+        if (!a.only_masked) fast_fp64<DIM3, OCC>(a, iblk, S, bi, bj, li + 8, lane, n_pp, n_rays);
         continue;
       }
-      const bool valid = (j < N) && (i < j);
+      const bool valid = (j < N) && (i < j) && (!a.only_masked || ((s_mask[li] >> lane) & 1u));
       const int64_t oi = a.orig ? (int64_t)a.orig[i] : i;
       const bool sw = valid && oi > oj;  // the reference casts from the lower caller index
       const int npi = a.np[i];

@@ -146,6 +146,7 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   w.dim3 = (m->dim == 2);
   w.pmax = T->pmax;
   if (o->fault_inject & RVF_FAULT_CLAIM) w.claim_retries = 0;
+  w.tables = T;
   w.fast_qb = o->fast_points;
   w.fast_groups = o->fast_row_groups;  // 0: by the tile count (wave_fast)
   // Meshes with occlusion run the occlusion kernels; the queue pipeline keeps
@@ -322,6 +323,16 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
     x.tmask = T->tmask.as<uint32_t>();
     x.segs = a.segs;
     if (!w.dim3) {
+      int rc = 0;
+      const size_t nt = (size_t)a.n_tiles;
+      if (T->tcls.bytes < nt && (rc = T->tcls.alloc(s, nt))) return rc;
+      if (T->tmask.bytes < nt * kTile * sizeof(uint32_t) && (rc = T->tmask.alloc(s, nt * kTile * sizeof(uint32_t))))
+        return rc;
+      cudaError_t e = cudaMemsetAsync(T->tcls.ptr, 0, nt, s->stream);
+      if (e == cudaSuccess) e = cudaMemsetAsync(T->tmask.ptr, 0, nt * kTile * sizeof(uint32_t), s->stream);
+      if (e != cudaSuccess) return cuda_err(e, "deferred tiles");
+      x.deferred = T->tcls.as<uint8_t>();
+      x.tmask = T->tmask.as<uint32_t>();
       // a computed hit of the reference's segment test (src/BVH.jl:265-322: |den| >= 1e-8, parameters strictly inside
       // (1e-8, 1 - 1e-8)) lies within about 2e-7 S^3 of both segments (S bounds every length)
       const double S = 2.0 * m->extent;
@@ -468,6 +479,50 @@ cudaError_t enqueue_chunk(Session* s, const WaveShape& sh, bool events) {
 }
 
 }  // namespace
+
+// The pairs of curves that the chunk's kernel deferred (tiles [t0, t0 + n) of a
+// request), in the queue pipeline.
+static int deferred_pairs(Session* s, const WaveReq& req, int64_t t0, int64_t n, bool use_graph, ChunkInfo* info) {
+  int rc = 0;
+  Tables* T = req.tables;
+  const size_t list_at = ((size_t)n + 255) & ~(size_t)255;
+  if ((rc = s->h_tiles.need(list_at + sizeof(int32_t) * n))) return rc;
+  const uint8_t* cls = s->h_tiles.as<uint8_t>();
+  int32_t* work = reinterpret_cast<int32_t*>(s->h_tiles.as<uint8_t>() + list_at);
+  cudaError_t e = cudaMemcpyAsync(s->h_tiles.ptr, T->tcls.as<uint8_t>() + t0, (size_t)n, cudaMemcpyDeviceToHost, s->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+  if (e != cudaSuccess) return cuda_err(e, "deferred tiles");
+  int64_t n_work = 0;
+  for (int64_t t = 0; t < n; ++t)
+    if (cls[t]) work[n_work++] = (int32_t)(t0 + t);
+  if (n_work == 0) return 0;
+  if (T->twork.bytes < sizeof(int32_t) * n_work && (rc = T->twork.alloc(s, sizeof(int32_t) * n_work))) return rc;
+  if ((e = cudaMemcpyAsync(T->twork.ptr, work, sizeof(int32_t) * n_work, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess)
+    return cuda_err(e, "deferred tile list upload");
+  WaveReq d = req;
+  d.occ_lists = false;
+  d.pa.tcls = T->tcls.as<uint8_t>();
+  d.pa.tmask = T->tmask.as<uint32_t>();
+  d.pa.work = T->twork.as<int32_t>();
+  d.pa.only_masked = true;
+  d.n_tiles = n_work;
+  d.claimed = 0;
+  WaveReq* one = &d;
+  while (!d.done()) {
+    const int64_t before = d.claimed;
+    ChunkInfo ci;
+    if ((rc = wave_chunk(s, &one, 1, use_graph, info ? &ci : nullptr))) return rc;
+    if (d.claimed == before) return no_progress(s);
+    if (info) {
+      info->ms_gen += ci.ms_gen;
+      info->ms_trace += ci.ms_trace;
+      info->ms_resolve += ci.ms_resolve;
+      info->rays_traced += ci.rays_traced;
+      info->kernels += ci.kernels;
+    }
+  }
+  return 0;
+}
 
 int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, ChunkInfo* info, int gen_bps,
                int trace_bps, double pp_budget, const std::function<void()>* on_launched) {
@@ -630,8 +685,10 @@ int wave_chunk(Session* s, WaveReq* const* reqs_in, int n_in, bool use_graph, Ch
   }
   // tiles are claimed in launch order: request r got min(claimed - base[r], its remaining tiles)
   const int64_t got = (int64_t)s->h_ctr[kCtrTile] / (fused ? ob.groups : 1);
+  const bool deferred = fused && !sh.dim3 && s->h_ctr[kCtrWalk] > 0;
   for (int r = 0; r < n; ++r) {
     const int64_t take = std::max<int64_t>(0, std::min<int64_t>(got - base[r], base[r + 1] - base[r]));
+    if (deferred && take > 0 && (rc = deferred_pairs(s, *reqs[r], reqs[r]->claimed, take, use_graph, info))) return rc;
     reqs[r]->claimed += take;
   }
   return 0;
