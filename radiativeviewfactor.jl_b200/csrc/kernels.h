@@ -475,6 +475,7 @@ struct McArgs {
   const TriD* tris;
   const SegD* segs;
   double cand_margin;  // curves: distance beyond which rounding cannot let a segment block a ray
+  int64_t n_segs;      //   obstruction segments
   float seg_slack;     //   FP32 rounding of the coordinates in the segment lists' hull tests
   const NodeF* nodesf;
   const int32_t* frontier;

@@ -922,7 +922,12 @@ cudaError_t launch_mc(const McArgs& a, int sm_count, cudaStream_t st) {
   const int64_t blocks = (int64_t)sm_count * per_sm, workers = a.dim3 ? 8 * blocks : blocks;
   b.rows = a.dim3 ? 4 : kTile;
   const int least = a.dim3 ? 1 : 8;
-  while (b.rows > least && a.tile_count * (kTile / b.rows) < 8 * workers) b.rows /= 2;
+  // Curves among more segments than a tile's list holds: the rows that walk the tree take
+  // hundreds of times as long as the others, so a claim is a row for each warp.  Cavities
+  // of 3,016 / 3,800 Line3 with 3,000 segments, 16 samples: 70 / 80 to 90 ms with whole tiles,
+  // 21 / 30 ms so (58 / 61 ms with a tree walk for each pair, before there were lists).
+  const bool uneven = !a.dim3 && occ && a.n_segs > kSegs;
+  while (b.rows > least && (uneven || a.tile_count * (kTile / b.rows) < 8 * workers)) b.rows /= 2;
   const int64_t tasks = a.tile_count * (kTile / b.rows), per_block = a.dim3 ? 8 : 1;
   const unsigned grid = (unsigned)std::min<int64_t>(blocks, (tasks + per_block - 1) / per_block);
   if (!a.dim3) {

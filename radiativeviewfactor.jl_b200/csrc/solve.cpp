@@ -135,6 +135,7 @@ void fill_mc_args(Session* s, rvf_mesh* m, const rvf_options* o, uint8_t* ray_lo
     const double S = 2.0 * m->extent;
     c.cand_margin = 1e-5 * S * S * S + std::ldexp(S, -16);
     c.seg_slack = (float)std::ldexp(m->extent, -20);
+    c.n_segs = m->n_obs;
     c.nodesf = occ ? m->nodesf.as<NodeF>() : nullptr;
     c.frontier = occ ? m->frontier.as<int32_t>() : nullptr;
     c.n_frontier = occ ? m->n_frontier : 0;
