@@ -438,8 +438,9 @@ int mesh_upload(Session* s, const rvf_mesh_desc* d, rvf_mesh** out) {
       for (int pass = 0; pass < 2; ++pass) {
         const std::vector<TriD>& src = pass == 0 ? tref : tgeo;
         std::vector<float> sat((size_t)T * 12);
-        std::vector<double> height;  // of the triangles that are not degenerate
+        std::vector<double> height, margin;  // of the triangles that are not degenerate
         height.reserve((size_t)T);
+        margin.reserve((size_t)T);
         for (int64_t k = 0; k < T; ++k) {
           const TriD& t = src[k];
           double l2 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0;
@@ -449,12 +450,15 @@ int mesh_upload(Session* s, const rvf_mesh_desc* d, rvf_mesh** out) {
             q3 += (t.e2[c] - t.e1[c]) * (t.e2[c] - t.e1[c]);
           }
           l2 = std::max(q1, std::max(q2, q3)) * (1.0 + 1e-9);
+          const double lx = std::min(std::sqrt(l2), S);
+          const double mt = 2.0 * 1.111e-6 * (65.0 * S * l2 + 40.0 * l2 * lx);
           const double cx = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1], cy = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2],
                        cz = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
           const double area = std::sqrt(cx * cx + cy * cy + cz * cz);
-          if (area > 1e-9 * l2) height.push_back(area / std::sqrt(l2));
-          const double lx = std::min(std::sqrt(l2), S);
-          const double mt = 2.0 * 1.111e-6 * (65.0 * S * l2 + 40.0 * l2 * lx);
+          if (area > 1e-9 * l2) {
+            height.push_back(area / std::sqrt(l2));
+            margin.push_back(mt);
+          }
           float* o = sat.data() + 12 * k;
           for (int c = 0; c < 3; ++c) {
             o[c] = (float)t.v0[c];
@@ -465,10 +469,13 @@ int mesh_upload(Session* s, const rvf_mesh_desc* d, rvf_mesh** out) {
           std::memcpy(&o[7], &t.group, 4);
           o[11] = 0.f;
         }
-        if (!height.empty()) {
-          std::nth_element(height.begin(), height.begin() + height.size() / 2, height.end());
-          m->tri_height[pass] = height[height.size() / 2];
-        }
+        auto median = [](std::vector<double>& v) {
+          if (v.empty()) return 0.0;
+          std::nth_element(v.begin(), v.begin() + v.size() / 2, v.end());
+          return v[v.size() / 2];
+        };
+        m->tri_height[pass] = median(height);
+        m->tri_margin[pass] = median(margin);
         if ((rc = upload(s, pass == 0 ? m->sat_ref : m->sat_geo, sat.data(), sizeof(float) * sat.size()))) return rc;
       }
       for (int pass = 0; pass < 2; ++pass) {

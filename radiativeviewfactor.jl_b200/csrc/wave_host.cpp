@@ -123,11 +123,15 @@ static int ensure_occ(Session* s, int64_t n_tiles, OccQ& q, int& grid) {
 //   FP64, 7 points, 1,728 Tri3, 10,800 triangles (0.93): 10.9 / 9.4; 4,800 Tri3, 4,800 (0.81): 41.0 / 47.4
 //   mixed, 13 points, 768 Tri3, 4,800 triangles (1.0): 6.6 / 3.8; 7 points, 30,000 Tri3, 2,352 (0.30): 198 / 232
 //   FP64, 7 points, 108 Tri3, 1,200 triangles (long 1.0): 1.23 / 0.72, the rows of few tiles one after another
-static bool occ_by_queue(bool mixed, bool geometric, int pmax, int64_t n_tiles, double wide, double lng) {
+// loose: the margin by which rounding can move a hit (it grows with the cube of the unit)
+// exceeds a tenth of the triangles' height, so that lists hold whole leaves.  4,800
+// Tri3, 1,728 triangles (long 0.1) at a scale of 1,000, 1 / 3 points, mixed: 9.3 / 6.9, 19.7 / 14.6.
+static bool occ_by_queue(bool mixed, bool geometric, bool loose, int pmax, int64_t n_tiles, double wide, double lng) {
   const bool few = n_tiles <= 64 && lng >= 0.9 && wide < 0.5;
   if (pmax == 1 && n_tiles <= 200) return wide >= 0.98;
   if (pmax <= 4) {
     if (few && pmax > 1) return true;
+    if (n_tiles > 64 && ((loose && lng >= 0.04) || (mixed && geometric && lng >= 0.08))) return true;
     if (mixed) return n_tiles > 64 && (wide >= (geometric ? 0.15 : 0.25) || lng >= 0.5);
     return wide >= (geometric ? 0.3 : 0.4);
   }
@@ -145,11 +149,11 @@ static bool occ_by_queue(bool mixed, bool geometric, int pmax, int64_t n_tiles, 
 // triangles, at scales of 1e-4 to 1e3 and offsets to 1e5), lists against the queue
 // pipeline: share 0.013, 1.3 to 2.3x as fast; 0.018, 0.55 to 1.2x; 0.035, 0.14 to 0.5x;
 // 0.35, 0.07 to 0.1x.  Rules of up to four points, which gain less: 0.0027, 1.1 to 1.6x;
-// 0.0037, 0.8 to 0.9x.
-static bool fp32_too_coarse(const rvf_mesh* m, bool geometric, int pmax) {
+// 0.0037, 0.8 to 0.9x.  Mixed precision with true vertices: 0.0027, 0.9 to 1.1x.
+static bool fp32_too_coarse(const rvf_mesh* m, bool mixed, bool geometric, int pmax) {
   const double h = m->tri_height[geometric ? 1 : 0];
   const double share = h > 0.0 ? std::ldexp(m->extent, -20) / h : 0.0;
-  return share >= (pmax <= 4 ? 3e-3 : 1.5e-2);
+  return share >= (mixed && geometric ? 2.5e-3 : pmax <= 4 ? 3e-3 : 1.5e-2);
 }
 
 int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8_t* ray_log, WaveReq& w,
@@ -171,7 +175,7 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   // 25-bit triangle indices.
   w.occ_lists = occ && !o->disable_tile_cull && !ray_log && !(o->fault_inject & RVF_FAULT_CLAIM) &&
             m->frontier.ptr && m->n_nodes < (1 << 24) && m->n_obs < (1 << 25) &&
-            !(w.dim3 && fp32_too_coarse(m, o->geometric_soup != 0, w.pmax));
+            !(w.dim3 && fp32_too_coarse(m, w.mixed, o->geometric_soup != 0, w.pmax));
   PairArgs& a = w.pa;
   a.N = N;
   a.nT = (N + kTile - 1) / kTile;
@@ -293,8 +297,10 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
         }
         w.row_end[(size_t)bi] = n_work;
       }
+      const int geo = o->geometric_soup ? 1 : 0;
       if (w.occ_lists && n_slow > 0 &&
-          occ_by_queue(w.mixed, o->geometric_soup != 0, a.pmax, a.n_tiles, (double)n_wide / n_slow, (double)n_long / n_slow)) {
+          occ_by_queue(w.mixed, o->geometric_soup != 0, m->tri_margin[geo] > 0.1 * m->tri_height[geo], a.pmax, a.n_tiles,
+                       (double)n_wide / n_slow, (double)n_long / n_slow)) {
         // the queue pipeline, which needs the masks: the same classes again, with them
         w.occ_lists = false;
         c.mask = T->tmask.as<uint32_t>();

@@ -34,3 +34,22 @@ def test_scales_and_offsets(rvf, orc, session, scale, offset, queue, geometric):
             assert_rel(np.where(same, 0.0, F), np.where(same, 0.0, Fo))
         elif offset == 0.0:
             assert np.max(np.abs(F - Fo)) <= 1e-6
+
+
+@pytest.mark.parametrize("scale,nquad,queue", [(1.0, 2, False), (1e3, 2, True), (1e3, 3, False)])
+def test_large_units(rvf, orc, session, scale, nquad, queue):
+    """Millimetres: the margin of the lists' triangle test exceeds the triangles, and rules of few points
+    among many leaves are taken by the queue pipeline (occ_by_queue)."""
+    from rvf_b200 import _abi
+    md = rvf.meshes.cube_enclosure(12, box_m=12)
+    md.coords[...] *= scale
+    md.group_tri_soup[7] = md.group_tri_soup[7] * scale
+    dm = _abi.DeviceMesh(session, rvf.mesh_desc_arrays(md, [7]))
+    try:
+        F = np.empty((md.n_elems,) * 2, order="F")
+        st = dm.solve(rvf.make_options(nquad, seed=0), F).as_dict()
+    finally:
+        dm.release()
+    assert (st["ms_resolve"] > 0.0) == queue
+    raw, area, _, _ = orc.solve_plain(orc.Mesh(md, [7]), nquad)
+    assert_rel(F, orc.f_from_raw(raw, area))
