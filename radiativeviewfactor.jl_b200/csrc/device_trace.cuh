@@ -163,10 +163,16 @@ __device__ __forceinline__ void buf_collect(const WarpScratch& ws, int b, int n,
 // (nodes(k) returns node k: GlobalNodes or SwizNodes)
 //   leaf(const Node&, int& first, int& count)
 //   prim(ws, owner, k) -> int  kHit / kMiss / kUnsure for owner's ray
-// Returns kHit (blocked), kMiss (visible) or kUnsure (FP32 only: some
-// decision of the walk was not certain and no certain hit was found).
+// Returns kHit (blocked), kMiss (visible) or kUnsure (FP32 only: a triangle
+// is or may be hit, but that or its leaf's box is not certain, and no certain hit was
+// found).  OPEN: an uncertain box is walked as a passed one: a leaf's box passes only if
+// every ancestor's does (box monotonicity, for the finite 1/d of an FP32 ray),
+// so the leaf's own test decides.  Rays that end on a face of the obstruction
+// touch its boxes there; without OPEN an uncertain box ends the walk (right
+// where most rays are uncertain: FP32 coordinates coarse beside the boxes).
 // ---------------------------------------------------------------------------
-template <typename Src, typename Pol, int L>
+constexpr int kOpenLeaf = 1 << 30;  // a collected leaf whose box test is not certain
+template <bool OPEN = false, typename Src, typename Pol, int L>
 __device__ __forceinline__ int trace_batch(bool have, const Src& nodes, int n_nodes, RayBankT<L>& ws, Pol& pol,
                                            TravCount& cnt) {
   static_assert(L <= 8, "leaf slot index is 3 bits");
@@ -187,19 +193,19 @@ __device__ __forceinline__ int trace_batch(bool have, const Src& nodes, int n_no
       const int s = pol.node(nd);
       int first, count;
       pol.leaf(nd, first, count);
-      if (s == kUnsure) {
+      if (s == kUnsure) ++cnt.unsure_slab;
+      if (!OPEN && s == kUnsure) {
         unsure = true;
-        ++cnt.unsure_slab;
         done = true;
-      } else if (s == kHit && count > 0) {
-        ws.first[nl][lane] = first;
+      } else if (s != kMiss && count > 0) {
+        ws.first[nl][lane] = s == kUnsure ? first | kOpenLeaf : first;
         counts |= (uint32_t)count << (4 * nl);
         total_own += count;
         ++nl;
         k = pol.miss(nd);
       } else {
         // miss links point forward (checked when the tree is uploaded), so k grows
-        k = (s == kHit) ? k + 1 : pol.miss(nd);
+        k = (s != kMiss) ? k + 1 : pol.miss(nd);
       }
       if (k >= n_nodes) done = true;
     }
@@ -226,9 +232,10 @@ __device__ __forceinline__ int trace_batch(bool have, const Src& nodes, int n_no
       if (t < total) {
         const int it = ws.item[t];
         const int o = it >> 6;
-        const int r = pol.prim(ws, o, ws.first[(it >> 3) & 7][o] + (it & 7), cnt);
-        if (r == kHit) ws.hit[o] = 1;
-        else if (r == kUnsure) ws.unsure[o] = 1;
+        const int at = ws.first[(it >> 3) & 7][o];
+        const int r = pol.prim(ws, o, (at & ~kOpenLeaf) + (it & 7), cnt);
+        if (r == kHit && !(at & kOpenLeaf)) ws.hit[o] = 1;
+        else if (r != kMiss) ws.unsure[o] = 1;
       }
     }
     __syncwarp();

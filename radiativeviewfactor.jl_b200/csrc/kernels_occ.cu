@@ -718,18 +718,8 @@ __global__ void __launch_bounds__(256, 2) k_occ_rest(const OccBatch* __restrict_
   }
 }
 
-// Whether the FP64 ray (i, p) -> (j, q) is blocked, with the reference's
-// arithmetic, the warp's lanes taking its list's leaves.  A ray without a list,
-// or with 1/d not finite, walks the tree (every lane the same walk).
-// Warp-uniform call and result.
-struct Blocked64 {
-  bool blocked, reached;  // reached: the ray passes the root box
-  uint32_t nodes, prims;  // the lane's tests
-};
-__device__ __noinline__ Blocked64 occ_blocked64(const OccArgs& t, int64_t i, int64_t j, int p, int q, bool sw,
-                                                const uint32_t* list, int n) {
-  const int lane = threadIdx.x & 31;
-  Blocked64 c{false, false, 0, 0};
+// The reference's ray (i, p) -> (j, q), or false when none is cast.
+__device__ __forceinline__ bool occ_ray64(const OccArgs& t, int64_t i, int64_t j, int p, int q, bool sw, RayD& R) {
   const int pm = t.pmax;
   double xi[3], xj[3];
 #pragma unroll
@@ -739,10 +729,28 @@ __device__ __noinline__ Blocked64 occ_blocked64(const OccArgs& t, int64_t i, int
   }
   const double rx = xj[0] - xi[0], ry = xj[1] - xi[1], rz = xj[2] - xi[2];
   const double r2 = (rx * rx + ry * ry) + rz * rz;
+  return sw ? make_ray(xj, -rx, -ry, -rz, r2, R) : make_ray(xi, rx, ry, rz, r2, R);
+}
+// Whether it passes the root box.
+__device__ __noinline__ bool occ_reaches64(const OccArgs& t, int64_t i, int64_t j, int p, int q, bool sw) {
   RayD R;
-  if (!(sw ? make_ray(xj, -rx, -ry, -rz, r2, R) : make_ray(xi, rx, ry, rz, r2, R))) return c;
-  if (!slab_d(t.nodes[0], R)) return c;
-  c.reached = true;
+  return occ_ray64(t, i, j, p, q, sw, R) && slab_d(t.nodes[0], R);
+}
+
+// Whether the FP64 ray (i, p) -> (j, q) is blocked, with the reference's
+// arithmetic, the warp's lanes taking its list's leaves.  A ray without a list,
+// or with 1/d not finite, walks the tree (every lane the same walk).
+// Warp-uniform call and result.
+struct Blocked64 {
+  bool blocked;
+  uint32_t nodes, prims;  // the lane's tests
+};
+__device__ __noinline__ Blocked64 occ_blocked64(const OccArgs& t, int64_t i, int64_t j, int p, int q, bool sw,
+                                                const uint32_t* list, int n) {
+  const int lane = threadIdx.x & 31;
+  Blocked64 c{false, 0, 0};
+  RayD R;
+  if (!occ_ray64(t, i, j, p, q, sw, R) || !slab_d(t.nodes[0], R)) return c;
   const bool finite = !R.zdir && isfinite(R.inv[0]) && isfinite(R.inv[1]) && isfinite(R.inv[2]);
   if (n >= 0 && finite) {
     for (int b = 0; b < n && !c.blocked; b += 32) {
@@ -796,7 +804,7 @@ __device__ __noinline__ int occ_walk32(const OccArgs& t, bool live, const RayF R
   pol.tris = t.trisf;
   TravCount tc;
   if (live) pol.store(ws, threadIdx.x & 31, gi, gj);
-  const int s = trace_batch(live, GlobalNodes<NodeF>{t.nodesf}, t.n_nodes, ws, pol, tc);
+  const int s = trace_batch<true>(live, GlobalNodes<NodeF>{t.nodesf}, t.n_nodes, ws, pol, tc);
   tests[0] += tc.nodes;
   tests[1] += tc.prims;
   tests[2] += tc.unsure_slab;
@@ -991,11 +999,11 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
             if (rok) {
               const int sr = slab_f(nodesf[0], R[u]);
               if (sr != kMiss) {
-                live[u] = sr == kHit;
-                if (!live[u]) st[u] = kUnsure;
+                // (a ray that may miss the root box: its leaves decide, whose boxes lie in it)
+                live[u] = true;
                 if (MIXED && !exact) in64[u] = true;  // a ray the root box may hold
-                // mixed: the rays with FP64 terms; FP64: those that pass the root box (the uncertain ones below)
-                n_traced += MIXED ? !exact : sr == kHit;
+                // mixed: the rays with FP64 terms; FP64: those that pass the root box
+                n_traced += (MIXED ? !exact : sr == kHit || occ_reaches64(t, i, j, p, q, sw)) ? 1 : 0;
                 n_us += sr == kUnsure ? 1 : 0;
               }
             } else {
@@ -1003,6 +1011,7 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
               in64[u] = true;
               n_bad += MIXED && !exact ? 1 : 0;
               n_rays64 += MIXED && !exact ? 1 : 0;
+              n_traced += !MIXED && occ_reaches64(t, i, j, p, q, sw) ? 1 : 0;
             }
           }
         }
@@ -1052,8 +1061,8 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
         // FP64 for the uncertain rays, one after another
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          if (live[u] && st[u] != kHit && doubt[u]) st[u] = kUnsure + 1;
-          for (uint32_t m = __ballot_sync(kFull, st[u] >= kUnsure); m; m &= m - 1u) {
+          if (live[u] && st[u] != kHit && doubt[u]) st[u] = kUnsure;
+          for (uint32_t m = __ballot_sync(kFull, st[u] == kUnsure); m; m &= m - 1u) {
             const int src = __ffs(m) - 1;
             const Blocked64 x = occ_blocked64(t, i, j, __shfl_sync(kFull, pp[u], src), __shfl_sync(kFull, qq[u], src), sw,
                                               list, ps.n);
@@ -1062,7 +1071,6 @@ __global__ void __launch_bounds__(256, WALK ? 3 : 2) k_occ_pairs(const OccBatch*
             if (lane == src) {
               ++n_unsure;
               n_rays64 += MIXED ? 1 : 0;
-              n_traced += !MIXED && st[u] == kUnsure && x.reached ? 1 : 0;
               st[u] = x.blocked ? kHit : kMiss;
             }
           }
