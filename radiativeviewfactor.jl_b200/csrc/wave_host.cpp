@@ -132,12 +132,12 @@ static bool occ_by_queue(bool mixed, bool geometric, bool loose, int pmax, int64
   if (pmax <= 4) {
     if (few && pmax > 1) return true;
     if (n_tiles > 64 && ((loose && lng >= 0.04) || (mixed && geometric && lng >= 0.08))) return true;
-    if (mixed) return n_tiles > 64 && (wide >= (geometric ? 0.15 : 0.25) || lng >= 0.5);
-    return wide >= (geometric ? 0.3 : 0.4);
+    if (mixed) return n_tiles > 64 && (wide >= (geometric ? 0.15 : 0.25) || lng >= 0.35);
+    return wide >= (geometric ? 0.3 : 0.4) || (geometric && n_tiles > 64 && lng >= 0.1);
   }
   if (pmax <= 8 && few) return true;
   if (!mixed) return pmax <= 8 ? wide >= 0.92 : pmax <= 16 && few && n_tiles <= 16;
-  return pmax <= 16 && n_tiles >= 100 && lng >= 0.5;
+  return pmax <= 16 && n_tiles >= 100 && lng >= 0.42;
 }
 
 // Whether FP32 coordinates (2^-20 of 1 + the largest coordinate) are too coarse for
