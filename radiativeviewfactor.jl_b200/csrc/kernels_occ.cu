@@ -24,15 +24,19 @@
 // usable list, or with an infinite 1/d, walks the tree.
 //
 // Measured on a B200, closed cube of 43,200 Tri3 with a box of 1,728 triangles,
-// 7 points (FP64 / mixed precision, one solve): lists 41 / 42 ms, rest 13 / 16
-// ms, pairs 90 / 105 ms, 144 / 163 ms together, bound by instruction issue
+// 7 points (FP64 / mixed precision, one solve): lists 43 / 43 ms, rest 13 / 16
+// ms, pairs 89 / 105 ms, 144 / 164 ms together, bound by instruction issue
 // (65-75% of the slots).  Of the pairs' time about 24 / 30 ms set the rays up,
 // 58 ms test lists, the rest tests uncertain rays again.  The queue pipeline
 // (kernels_wave.cu), which also needs the classification's pair masks (36 ms), took
 // 310 / 224 ms for the same tiles: a record per ray and a slot and list per pair
 // through global memory, read back with dependent loads at 12 to 15 of 32 active
-// lanes.
-// Measured and not kept: all three steps in one kernel, lane = (pair, q) (284 /
+// lanes.  Where lists do not hold a tile (fine obstructions) or FP32 is too coarse that
+// pipeline is the faster one and takes the solve (wave_host.cpp: occ_by_queue,
+// fp32_too_coarse).
+// Measured and not kept: the uncertain rays of a pass tested in FP64 a lane each
+// instead of one after another (axis-aligned meshes, 9 points, mixed: 16.5 -> 14.3 ms;
+// the closed cube 216.3 -> 223.2 ms: registers of the kernel around it); all three steps in one kernel, lane = (pair, q) (284 /
 // 311 ms: 16 warps per SM cannot hide the list building's latency, four pairs'
 // lists differ in length); the (ray, triangle) tests packed into full warps
 // through shared memory (144 / 190 ms of pair kernel); the passing rays of a

@@ -118,7 +118,7 @@ static int ensure_occ(Session* s, int64_t n_tiles, OccQ& q, int& grid) {
 // or more.  Both sides were measured over 1,232 solves (12 to 30,000 elements of
 // every family, centred boxes of 12 to 10,800 triangles, rules of 1 to 64 points):
 // with lists alone 131 of them were slower than the queue pipeline had been, by up
-// to 1.8x; with these lines 12, by up to 1.07x.  Examples (ms, lists / queue; wide):
+// to 1.8x; with these lines 3, by up to 1.03x.  Examples (ms, lists / queue; wide):
 //   FP64, 1 point, 3,750 Quad4, 4,800 triangles (0.94): 8.5 / 4.5; 10,800 Tri3, 2,352 (0.46): 20.2 / 17.4
 //   FP64, 7 points, 1,728 Tri3, 10,800 triangles (0.93): 10.9 / 9.4; 4,800 Tri3, 4,800 (0.81): 41.0 / 47.4
 //   mixed, 13 points, 768 Tri3, 4,800 triangles (1.0): 6.6 / 3.8; 7 points, 30,000 Tri3, 2,352 (0.30): 198 / 232
