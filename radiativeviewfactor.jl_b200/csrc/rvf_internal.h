@@ -165,6 +165,7 @@ struct rvf_mesh {
   float sat_em = 0.f;
   double extent = 1.0;                        // 1 + max |coordinate| of the mesh and the soup
   double max_coord = 0.0;                     // max |coordinate| of the mesh's nodes
+  double aligned = 0.0;                       // share of element pairs aligned with a coordinate axis
   double tri_height[2] = {0.0, 0.0};          // median least height of the soup's triangles (read as the reference, true)
   double tri_margin[2] = {0.0, 0.0};          //   and median margin of the lists' triangle test
   int n_nodes = 0;

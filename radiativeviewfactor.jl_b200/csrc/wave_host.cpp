@@ -156,6 +156,19 @@ static bool fp32_too_coarse(const rvf_mesh* m, bool mixed, bool geometric, int p
   return share >= (mixed && geometric ? 2.5e-3 : pmax <= 4 ? 3e-3 : 1.5e-2);
 }
 
+// Whether a mixed solve has many rays with a direction component next to zero, which
+// FP32 cannot certify and the pair kernel takes to FP64 one after another, the tree's
+// walk for each: structured meshes along the axes (1.5 to 12% of the pairs aligned; nodes
+// displaced by 0.3 of an edge, 0.1%) under the obstruction's true vertices, where most
+// pairs are blockable.  Lists against the queue pipeline, ms, 9 points: 9,600 Quad4
+// 70.6 / 45.7, 5,000 Quad4 in two plates 27.4 / 18.3, 1,536 Quad8 3.48 / 2.54; 4 points,
+// 25.5 / 21.1, 10.3 / 9.2 and 1.46 / 1.28; 13 points, 3,072 Tri3 14.8 / 11.5.  At 16 the
+// lists win again where few rays are traced: 55.0 / 74.9 in the plates (7.1 / 6.3 for
+// 1,536 Quad4 in a cube), at 25 both are equal; 600 Quad4, 4 points, 0.62 / 0.66.
+static bool fp64_rays_many(const rvf_mesh* m, bool mixed, bool geometric, int pmax) {
+  return mixed && geometric && pmax > 1 && pmax < 16 && m->aligned >= 0.005;
+}
+
 int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8_t* ray_log, WaveReq& w,
                  int64_t* n_kernels) {
   const int64_t N = m->N;
@@ -175,7 +188,8 @@ int wave_prepare(Session* s, rvf_mesh* m, Tables* T, const rvf_options* o, uint8
   // 25-bit triangle indices.
   w.occ_lists = occ && !o->disable_tile_cull && !ray_log && !(o->fault_inject & RVF_FAULT_CLAIM) &&
             m->frontier.ptr && m->n_nodes < (1 << 24) && m->n_obs < (1 << 25) &&
-            !(w.dim3 && fp32_too_coarse(m, w.mixed, o->geometric_soup != 0, w.pmax));
+            !(w.dim3 && (fp32_too_coarse(m, w.mixed, o->geometric_soup != 0, w.pmax) ||
+                         fp64_rays_many(m, w.mixed, o->geometric_soup != 0, w.pmax)));
   PairArgs& a = w.pa;
   a.N = N;
   a.nT = (N + kTile - 1) / kTile;

@@ -31,3 +31,27 @@ def test_route(rvf, orc, session, family, m, box_m, nquad, precision, geometric,
         assert_rel(F, Fo)
     else:
         assert np.max(np.abs(F - Fo)) <= 1e-6
+
+
+@pytest.mark.parametrize("family,m,jitter,nquad,precision,geometric,queue", [
+    ("quad4", 12, 0.0, 3, "mixed", True, True), ("tri3", 9, 0.0, 2, "mixed", True, True),
+    ("quad", 8, 0.0, 3, "mixed", True, True), ("quad4", 12, 0.3, 3, "mixed", True, False),
+    ("quad4", 12, 0.0, 3, "mixed", False, False), ("quad4", 12, 0.0, 3, "fp64", True, False),
+    ("quad4", 12, 0.0, 4, "mixed", True, False)])
+def test_route_along_the_axes(rvf, orc, session, family, m, jitter, nquad, precision, geometric, queue):
+    """Structured meshes along the axes (fp64_rays_many), whose rays FP32 often cannot certify."""
+    from rvf_b200 import _abi
+    md = rvf.meshes.cube_enclosure(m, family=family, box_m=3, jitter=jitter)
+    dm = _abi.DeviceMesh(session, rvf.mesh_desc_arrays(md, [7]))
+    try:
+        F = np.empty((md.n_elems,) * 2, order="F")
+        st = dm.solve(rvf.make_options(nquad, precision=precision, geometric_soup=geometric, seed=0), F).as_dict()
+    finally:
+        dm.release()
+    assert (st["ms_resolve"] > 0.0) == queue
+    raw, area, _, cnt = orc.solve_plain(orc.Mesh(md, [7]), nquad, geometric=geometric)
+    Fo = orc.f_from_raw(raw, area)
+    if precision == "fp64":
+        assert_rel(F, Fo)
+    else:
+        assert np.max(np.abs(F - Fo)) <= 1e-6
